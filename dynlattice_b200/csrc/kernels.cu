@@ -16,21 +16,32 @@ __global__ void k_clear5(double *p) {
   if (threadIdx.x < 5) p[threadIdx.x] = 0.0;
 }
 
+// One warp: the running sum over the steps in their order, 32 steps loaded at
+// a time (a thread that walks the steps by itself waits for memory at each).
 __global__ void k_finish_wext(double *wstep, int n, double *wext_total, SampleSpec smp, int64_t step0,
                               int64_t sample_base, double *last_energy) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const int lane = threadIdx.x & 31;
   double acc = *wext_total;
-  for (int s = 0; s < n; ++s) {
-    acc += wstep[s];
-    wstep[s] = 0.0;
+  for (int s0 = 0; s0 < n; s0 += 32) {
+    const int s = s0 + lane;
+    const double w = s < n ? wstep[s] : 0.0;
+    if (s < n) wstep[s] = 0.0;
+    double mine = 0.0;
+    const int m = n - s0 < 32 ? n - s0 : 32;
+    for (int i = 0; i < m; ++i) {
+      acc += __shfl_sync(0xffffffffu, w, i);
+      if (i == lane) mine = acc;
+    }
     const int64_t step = step0 + s + 1;
-    if (smp.every > 0 && step % smp.every == 0) {
+    if (s < n && smp.every > 0 && step % smp.every == 0) {
       const int64_t idx = sample_base + step / smp.every - step0 / smp.every - 1;
-      if (idx < smp.capacity) smp.energy[idx * 5 + 3] = acc;
+      if (idx < smp.capacity) smp.energy[idx * 5 + 3] = mine;
     }
   }
-  *wext_total = acc;
-  last_energy[3] = acc;
+  if (lane == 0) {
+    *wext_total = acc;
+    last_energy[3] = acc;
+  }
 }
 
 
@@ -153,6 +164,14 @@ KernelSet aot_kernels(bool plastic) {
   return plastic ? aot_set<T, YieldInterp>() : aot_set<T, ElasticOnly>();
 }
 
+// Models of at most this many elements, nodes and pairs run in one block, whose
+// own barrier then replaces the grid's: two grid barriers are 3.5 us of a step.
+// FP64 rods, us per step, several blocks against one: 33 nodes 8.7 / 5.3, 128
+// nodes 10.2 / 5.8, 249 nodes (two items per thread) 9.3 / 8.6; an elastoplastic
+// 2^3 BCC lattice (163 nodes, 128 elements) 14.0 / 9.6.  Above that the one SM's
+// FP64 units and the items each thread walks cost what the barriers did.
+constexpr int kSoloWork = 256;
+
 template <class T>
 cudaError_t launch_steps(const KernelSet &ks, const DevModel<T> &m, const SampleSpec &smp, const StepCtx &c,
                          int mode, GridBarrier *bar, cudaStream_t s) {
@@ -170,9 +189,14 @@ cudaError_t launch_steps(const KernelSet &ks, const DevModel<T> &m, const Sample
     // which keeps the grid barriers short
     const int work = std::max(std::max(m.E, m.N), m.n_pairs);
     int tpb = ks.tpb_override > 0 ? ks.tpb_override : threads_for(work);
-    if (tpb == 256) tpb = ext ? ks.full_threads_x : ks.full_threads;
+    if (ks.tpb_override <= 0 && work <= kSoloWork) {
+      tpb = 32;
+      while (tpb < work && tpb < 128) tpb *= 2;
+    } else if (tpb == 256) {
+      tpb = ext ? ks.full_threads_x : ks.full_threads;
+    }
     const int ci = tpb == 32 ? 0 : (tpb == 64 ? 1 : (tpb == 128 ? 2 : 3));
-    const int want = std::max(1, (work + tpb - 1) / tpb);
+    const int want = ks.tpb_override <= 0 && work <= kSoloWork ? 1 : std::max(1, (work + tpb - 1) / tpb);
     // a launch of one step reports its energies: the kernel with that known
     const bool one = !ext && c.nsteps == 1 && ks.persistent1 && ks.persist_cap1[ci] > 0;
     const int cap = ext ? ks.persist_cap_x[ci] : (one ? ks.persist_cap1[ci] : ks.persist_cap[ci]);

@@ -984,11 +984,15 @@ __device__ __forceinline__ void node_update(const DevModel<T> &m, int n, int64_t
 // ---------------------------------------------------------------------------
 // grid barrier with a bounded wait
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned *p) {
   unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+
+// release and acquire at gpu scope (lighter than __threadfence(), which is
+// sequentially consistent)
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -1000,30 +1004,35 @@ __device__ __forceinline__ unsigned long long global_ns() {
 struct BarrierState {
   unsigned add0;                // block 0's arrival increment
   unsigned long long limit_ns;  // bound of one wait
+  bool solo;                    // a launch of one block: its own barrier is the grid's
 };
 __device__ __forceinline__ BarrierState barrier_begin(const GridBarrier *b) {
   const unsigned expect = gridDim.x + b->phantom;
   const unsigned lim = b->limit_us;
-  return BarrierState{0x80000000u - (expect - 1u), lim ? 1000ull * lim : 2000000000ull};
+  return BarrierState{0x80000000u - (expect - 1u), lim ? 1000ull * lim : 2000000000ull, expect == 1u};
 }
 
 // Returns false when the barrier was abandoned (its wait ran out here or in
 // another block).  One atomic per block: the arrival (after a fence that
 // publishes the block's writes) returns the word before it; the block then
-// polls with acquire loads until bit 31 differs from that value.
+// polls until bit 31 differs from that value, and one fence afterwards makes
+// the other blocks' writes visible.  The polls are relaxed loads: an acquire
+// load drops the SM's L1 each time, under the warps of the SM's other block
+// that are still working.
 static __device__ bool grid_barrier(GridBarrier *b, const BarrierState &bs, uint32_t *err) {
   __shared__ int s_ok;
   __syncthreads();
+  if (bs.solo) return true;
   if (threadIdx.x == 0) {
     int ok = 1;
     const unsigned inc = blockIdx.x == 0 ? bs.add0 : 1u;
-    __threadfence();  // the block's writes (ordered by __syncthreads) before the arrival
+    fence_gpu();  // the block's writes (ordered by __syncthreads) before the arrival
     const unsigned old = atomicAdd(&b->count, inc);
     unsigned polls = 0;
     unsigned long long t0 = 0;
-    while (((ld_acquire(&b->count) ^ old) & 0x80000000u) == 0u) {
+    while (((ld_relaxed(&b->count) ^ old) & 0x80000000u) == 0u) {
       if ((++polls & 63u) == 0u) {  // the abort flag and the clock now and then
-        if (ld_acquire(&b->abort)) {
+        if (ld_relaxed(&b->abort)) {
           ok = 0;
           break;
         }
@@ -1038,7 +1047,7 @@ static __device__ bool grid_barrier(GridBarrier *b, const BarrierState &bs, uint
         }
       }
     }
-    __threadfence();
+    fence_gpu();
     s_ok = ok;
   }
   __syncthreads();
