@@ -56,8 +56,8 @@ __device__ __forceinline__ void adj_node_one(const DevModel<T> &m, const AdjCtx<
   in.R = Q4<double>{r0.x, r0.y, r0.z, r0.w};
   double v1[6];
   for (int k = 0; k < 6; ++k) {
-    in.v[k] = m.tp_vel[(s0 * 6 + k) * N + n];
-    v1[k] = m.tp_vel[(s1 * 6 + k) * N + n];
+    in.v[k] = m.tp_vel[s0 * 6 * tiles32(N) + vel_ix(n, k)];
+    v1[k] = m.tp_vel[s1 * 6 * tiles32(N) + vel_ix(n, k)];
   }
   in.mass = m.mass[n];
   const auto Pq = m.iframe[n];
@@ -183,15 +183,16 @@ __global__ void __launch_bounds__(256) k_adj_elem(const __grid_constant__ DevMod
       }
       double ldiss = 0.0;
       if (plastic) {
-        const size_t o6 = s0 * G * 6 * E, oh = s0 * G * nh * E;
+        const size_t E32 = s0 * tiles32(E) * G;
+        const T *const th = m.tp_hist + E32 * m.hs, *const te = m.tp_epsc + E32 * 6;
         for (int q = 0; q < 6; ++q) {
-          gi.ep[q] = m.tp_ep[o6 + (g * 6 + q) * E + e];
-          gi.epsc[q] = m.tp_epsc[o6 + (g * 6 + q) * E + e];
+          gi.ep[q] = th[hist_ix<T>(G, m.hs, e, g, q)];
+          gi.epsc[q] = te[epsc_ix(G, e, g, q)];
           lh.ep[q] = a.lep[(g * 6 + q) * E + e];
           lh.epsc[q] = a.lepsc[(g * 6 + q) * E + e];
         }
         for (int q = 0; q < nh; ++q) {
-          gi.al[q] = m.tp_al[oh + (g * nh + q) * E + e];
+          gi.al[q] = th[hist_ix<T>(G, m.hs, e, g, 6 + q)];
           lh.al[q] = a.lal[(g * nh + q) * E + e];
         }
         ldiss = a.w_diss * adj_gw(G, g) * 0.5 * in.L0;

@@ -140,8 +140,10 @@ __global__ void k_closed(const double4 *pos, const int2 *conn, const int2 *pairs
 
 __global__ void k_max_speed(const double *vel, int N, unsigned long long *out) {
   double m = 0.0;
-  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x)
-    m = fmax(m, sqrt(vel[n] * vel[n] + vel[N + n] * vel[N + n] + vel[2 * N + n] * vel[2 * N + n]));
+  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
+    const double a = vel[vel_ix(n, 0)], b = vel[vel_ix(n, 1)], c = vel[vel_ix(n, 2)];
+    m = fmax(m, sqrt(a * a + b * b + c * c));
+  }
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) atomicMax(out, __double_as_longlong(m));
 }

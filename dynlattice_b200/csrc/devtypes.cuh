@@ -4,7 +4,7 @@
 // Nodes (renumbered along a Morton curve so that elements gather neighbours):
 //   pos   double4[N]    x, y, z, (unused)          -- FP64 state
 //   rot   double4[N]    unit quaternion w,x,y,z    -- FP64 state
-//   vel   double[6][N]  SoA, translational + spatial angular velocity
+//   vel   double2[3][32] per 32 nodes (vel_ix): translational + spatial angular velocity
 //   mass  double[N]     translational lumped mass
 //   iframe T4[N]        principal frame P of the rotational inertia S = P D P^T
 //   idiag  T4[N]        D (3 principal moments), w = unused; idinv: 1/D
@@ -18,8 +18,12 @@
 //   g0    T[G*3][E]     Gamma0 - e3 ; k0 T[G*3][E]: K0  (initStrain_)
 //   C     T[6][E]       diag(GkA, GkA, EA, EI1, EI2, GJ)
 //   ec    T[2][E]       element variables of yield expressions: radius, area
-//   ep    T[G*6][E], alpha T[G*nh][E], epsc T[G*6][E]: plastic strain,
-//                       hardening parameters, committed total strain
+//   hist  per Gauss point plastic strain (6) and hardening parameters (nh), in
+//                       16-byte vectors (hist_ix); epsc: committed total strain
+//                       (6), in pairs (epsc_ix); both for tiles of 32 elements
+//   erec  16-byte vectors, tiles of 32 elements: everything constant about a
+//                       two-node element that a step reads (ElemRecIx); nrec the
+//                       same per node (NodeRecIx)
 //   ediss double[G][E]  dissipated energy per Gauss point
 //   eslot int2[E]       slots of the element's two ends
 //   ef    T[2E][6]      end forces in node-ordered slots: an element writes
@@ -74,6 +78,69 @@ struct Vec4 {
 template <>
 struct Vec4<float> {
   using type = float4;
+};
+
+// 16-byte vectors of T: the step kernels load and store records of them, a
+// warp's 32 items side by side (one instruction moves 512 contiguous bytes, and
+// the vectors of one record are constant offsets apart).
+template <class T>
+struct Vec16 {
+  using type = double2;
+  static constexpr int n = 2;
+};
+template <>
+struct Vec16<float> {
+  using type = float4;
+  static constexpr int n = 4;
+};
+#if defined(__CUDACC__)
+#define DL_HDI __host__ __device__ __forceinline__
+#else
+#define DL_HDI inline
+#endif
+// position of scalar s of item i's record of nv vectors
+template <class T>
+DL_HDI size_t rec_ix(int nv, int i, int s) {
+  constexpr int n = Vec16<T>::n;
+  return ((static_cast<size_t>(i >> 5) * nv + s / n) * 32 + (i & 31)) * n + s % n;
+}
+// scalars of the history record of one Gauss point: plastic strain,
+// hardening parameters, padded to whole vectors
+template <class T>
+DL_HDI int hist_scalars(int nh) {
+  constexpr int n = Vec16<T>::n;
+  return (6 + nh + n - 1) / n * n;
+}
+// scalar k of Gauss point g of element e in the history records (hs scalars a point)
+template <class T>
+DL_HDI size_t hist_ix(int G, int hs, int e, int g, int k) {
+  return rec_ix<T>(G * hs / Vec16<T>::n, e, g * hs + k);
+}
+// strain component k (pairs of T, tiles of 32 elements)
+DL_HDI size_t epsc_ix(int G, int e, int g, int k) {
+  return ((static_cast<size_t>(e >> 5) * (G * 3) + g * 3 + k / 2) * 32 + (e & 31)) * 2 + k % 2;
+}
+// velocity component k of node n
+DL_HDI size_t vel_ix(int n, int k) { return ((static_cast<size_t>(n >> 5) * 3 + k / 2) * 32 + (n & 31)) * 2 + k % 2; }
+// items of whole tiles
+DL_HDI int tiles32(int n) { return (n + 31) & ~31; }
+
+// Scalars of an element's record: one vector of four ints (nodes, end-force
+// slots), then Lambda_N of both ends, C, radius, area, K0 (the same at every
+// Gauss point of a two-node element), L0, 1/L0 (a double) and Gamma0 - e3 per point.
+template <class T>
+struct ElemRecIx {
+  static constexpr int ints = 0, qN = 16 / sizeof(T), C = qN + 8, ec = C + 6, k0 = ec + 2, L0 = k0 + 3, invL0 = L0 + 1,
+                       g0 = invL0 + 8 / sizeof(T);
+  DL_HDI static constexpr int vecs(int G) { return (g0 + 3 * G + Vec16<T>::n - 1) / Vec16<T>::n; }
+};
+// Scalars of a node's record: end-force slots and boundary terms [first, last)
+// (four ints; a node whose terms all set accelerations to zero has -1 - mask of
+// its held DOFs in place of the first term, one without terms -1), principal frame P, moments D, 1/D, 1/mass (a double).
+template <class T>
+struct NodeRecIx {
+  static constexpr int ints = 0, P = 16 / sizeof(T), imass = P + 4, D = imass + 8 / sizeof(T), Dinv = D + 3;
+  static constexpr int vecs = (Dinv + 3 + Vec16<T>::n - 1) / Vec16<T>::n;
 };
 
 // Expression program in device memory
@@ -133,9 +200,11 @@ struct DevModel {
   const T *k0 = nullptr;
   const T *C = nullptr;
   const T *ec = nullptr;
-  T *ep = nullptr;
-  T *alpha = nullptr;
+  int hs = 0;              // scalars of a point's history record (hist_scalars)
+  T *hist = nullptr;
   T *epsc = nullptr;
+  const typename Vec16<T>::type *erec = nullptr;  // null for elements of 3 or 4 nodes
+  const typename Vec16<T>::type *nrec = nullptr;
   double *ediss = nullptr;
   T *ef = nullptr;
   // elements of 3 or 4 nodes (nen > 2; two-node elements use conn/eslot):
@@ -214,12 +283,11 @@ struct DevModel {
   double *fint_last = nullptr;  // [6][N] internal force of the last step of a launch (GroupOutput "resp")
   // state tape of the adjoint's recomputation (null in plain runs): slot
   // s = step - tp_step0 holds the state after that step; tp_pos/tp_rot [slot][N],
-  // tp_vel [slot][6][N], tp_ep/tp_epsc [slot][G*6*E], tp_al [slot][G*nh*E]
+  // tp_vel, tp_hist and tp_epsc the arrays vel, hist and epsc per slot
   double4 *tp_pos = nullptr;
   double4 *tp_rot = nullptr;
   double *tp_vel = nullptr;
-  T *tp_ep = nullptr;
-  T *tp_al = nullptr;
+  T *tp_hist = nullptr;
   T *tp_epsc = nullptr;
   int64_t tp_step0 = 0;
   // per-step sum of one internal-force component over a node group (null in
@@ -251,8 +319,8 @@ struct MilneCtl {
 template <class T>
 struct MilneDev {
   double4 *pos_pre, *rot_pre;  // predicted, then corrected node state
-  double *vel_pre;             // [6][N]
-  T *ep_new, *alpha_new, *epsc_new;  // history of the corrector's force evaluation
+  double *vel_pre;             // as vel
+  T *hist_new, *epsc_new;  // history of the corrector's force evaluation
   double *ediss_new;
   double *partial;             // [gridDim][3] per-block sums of the error norms and the external work
   MilneCtl *ctl;
@@ -303,6 +371,17 @@ struct GridBarrier {
   unsigned int phantom;
   unsigned int abort;
   unsigned int limit_us;
+};
+
+// Which elements and nodes each block of a launch takes in the
+// one-barrier step kernel (local.cuh).
+struct LocalPlan {
+  int chunk = 0;                     // elements per block: block b takes [b chunk, (b + 1) chunk)
+  int cap = 0;                       // most node copies of a block
+  int recs = 0;                      // whether the blocks keep their elements' records in shared memory
+  const int32_t *node_ptr = nullptr;  // [blocks + 1] runs of nodes
+  const int32_t *nodes = nullptr;     // node, sign bit set where this block owns it
+  const uint32_t *ends = nullptr;     // [E] the two end nodes as copies of the element's block (16 bits each)
 };
 
 struct StepCtx {

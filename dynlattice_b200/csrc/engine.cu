@@ -21,6 +21,7 @@
 
 #include "../../include/dynlattice.h"
 #include "engine.hpp"
+#include "local.cuh"
 #include "jit.hpp"
 #include "noalloc.hpp"
 #include "output.hpp"
@@ -69,7 +70,7 @@ void trim_retained_pool() { DL_CUDA(cudaMemPoolTrimTo(retained_pool(), 0)); }
 // and read by the reverse sweep: node positions, rotations, velocities and
 // the plastic history of every Gauss point.
 struct StateTape {
-  PoolBuf pos, rot, vel, ep, al, epsc;
+  PoolBuf pos, rot, vel, hist, epsc;
 };
 
 template <class T>
@@ -163,12 +164,12 @@ struct Engine final : EngineBase {
   using T4 = typename Vec4<T>::type;
   DevModel<T> m;
   DevBuf pos, rot, vel, mass, imass, iframe, idiag, idinv, slot_ptr, bc_ptr, bc, madd;
-  DevBuf conn, eslot, invL0, L0, qN, g0, k0, C, ec, ep, alpha, epsc, ediss, ef, cstamp;
+  DevBuf conn, eslot, invL0, L0, qN, g0, k0, C, ec, hist, epsc, ediss, ef, cstamp, erec, nrec;
   DevBuf conn_n, eslot_n, shp, s0_n;  // elements of 3 or 4 nodes
   DevBuf yops, yconsts, gops, gconsts, gouts;
   DevBuf err, wext_dev, scales, wstep, energy_slots, barrier;
   // adjoint: checkpoints, tape of one segment, adjoint state, objective group
-  PoolBuf ck_pos, ck_rot, ck_vel, ck_ep, ck_al, ck_epsc, ck_ediss;
+  PoolBuf ck_pos, ck_rot, ck_vel, ck_hist, ck_epsc, ck_ediss;
   // state tapes: two sets, so that the recomputation of one checkpoint
   // segment overlaps the reverse sweep over the next one
   StateTape tape[2];
@@ -205,7 +206,7 @@ struct Engine final : EngineBase {
   // MilneDevice predictor-corrector (dl_set_integrator)
   dl_integrator_desc integ{};
   MilneDev<T> md{};
-  DevBuf mi_pos, mi_rot, mi_vel, mi_ep, mi_al, mi_epsc, mi_ediss, mi_partial, mi_ctl, mi_ops, mi_consts, mi_outs;
+  DevBuf mi_pos, mi_rot, mi_vel, mi_hist, mi_epsc, mi_ediss, mi_partial, mi_ctl, mi_ops, mi_consts, mi_outs;
   DevBuf s_times;
   double cur_dt = 0.0;      // the time step of the next step
   int64_t rejected = 0;
@@ -234,7 +235,12 @@ struct Engine final : EngineBase {
     // nodes
     upload(pos, h.pos);
     upload(rot, h.rot);
-    upload(vel, h.vel);
+    {
+      std::vector<double> v(static_cast<size_t>(tiles32(N)) * 6, 0.0);
+      for (int n = 0; n < N; ++n)
+        for (int k = 0; k < 6; ++k) v[vel_ix(n, k)] = h.vel[static_cast<size_t>(k) * N + n];
+      upload(vel, v);
+    }
     upload(mass, h.mass);
     upload_as<T>(iframe, h.iframe);
     upload_as<T>(idiag, h.idiag);
@@ -309,16 +315,15 @@ struct Engine final : EngineBase {
       for (int g = 0; g < 4; ++g) m.Nq[a][g] = h.Nq[a][g];
     if (h.plastic) {
       const size_t NG = static_cast<size_t>(E) * G;
-      ep.alloc(NG * 6 * sizeof(T));
-      DL_CUDA(cudaMemset(ep.p, 0, ep.bytes));
-      alpha.alloc(NG * std::max(1, h.nh) * sizeof(T));
-      DL_CUDA(cudaMemset(alpha.p, 0, alpha.bytes));
-      epsc.alloc(NG * 6 * sizeof(T));
+      const size_t NG32 = static_cast<size_t>(tiles32(E)) * G;
+      m.hs = hist_scalars<T>(h.nh);
+      hist.alloc(NG32 * m.hs * sizeof(T));
+      DL_CUDA(cudaMemset(hist.p, 0, hist.bytes));
+      epsc.alloc(NG32 * 6 * sizeof(T));
       DL_CUDA(cudaMemset(epsc.p, 0, epsc.bytes));
       ediss.alloc(NG * sizeof(double));
       DL_CUDA(cudaMemset(ediss.p, 0, ediss.bytes));
-      m.ep = ep.as<T>();
-      m.alpha = alpha.as<T>();
+      m.hist = hist.as<T>();
       m.epsc = epsc.as<T>();
       m.ediss = ediss.as<double>();
       upload(yops, h.yield.ops);
@@ -339,6 +344,7 @@ struct Engine final : EngineBase {
       m.max_iter = h.max_iter;
       m.prec = T(h.prec);
     }
+    upload_records();
     ef.alloc(static_cast<size_t>(E) * 6 * h.nen * sizeof(T));  // one 6-value slot per element node
     DL_CUDA(cudaMemset(ef.p, 0, ef.bytes));
     m.ef = ef.as<T>();
@@ -427,7 +433,134 @@ struct Engine final : EngineBase {
       const KernelSet *ks = jit_kernels(code, sizeof(T) == 4, &jit_log);
       if (ks) kernels = *ks;
     }
+    plan_local();
     set_sampling(0, {}, 0);
+  }
+
+  // The one-barrier kernel's share-out of elements and node copies over the
+  // blocks.  One block per SM while the elements of a block stay below its
+  // threads, two above that; a model whose copies do not fit, or that uses what
+  // the kernel does not cover, keeps the two-barrier kernels (blocks = 0).
+  LocalLaunch local;
+  DevBuf local_ptr, local_nodes, local_ends;
+  void plan_local() {
+    const HostLattice &h = *host;
+    const bool ext = contact_on || joint_on || m.n_plates > 0 || h.lumped || h.ties || h.nen != 2;
+    if (ext || !kernels.local[0]) return;
+    const int E = h.E;
+    int sms = 0;
+    DL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int most = kernels.local_threads;
+    int per_sm = 1, chunk = E;
+    if (std::max(h.N, E) > kSoloWork) {
+      per_sm = E > sms * most ? 2 : 1;
+      chunk = (E + per_sm * sms - 1) / (per_sm * sms);
+      chunk = std::max(32, (chunk + 7) / 8 * 8);
+    }
+    const int blocks = (E + chunk - 1) / chunk;
+    if (static_cast<size_t>(chunk) * sizeof(double) * LocalShape<T>::row / 2 > 232448) return;  // copies >= half the elements
+    std::vector<int32_t> ptr(blocks + 1, 0), nodes;
+    std::vector<uint32_t> ends(E);
+    std::vector<int32_t> at(h.N, -1), seen(h.N, -1);
+    int cap = 0;
+    for (int b = 0; b < blocks; ++b) {
+      const int first = static_cast<int>(nodes.size());
+      const int e1 = std::min(E, (b + 1) * chunk);
+      for (int e = b * chunk; e < e1; ++e)
+        for (int a = 0; a < 2; ++a) {
+          const int n = h.conn[2 * e + a];
+          if (seen[n] == b) continue;
+          nodes.push_back(seen[n] < 0 ? static_cast<int32_t>(static_cast<uint32_t>(n) | 0x80000000u) : n);
+          seen[n] = b;
+        }
+      // nodes with equally many slots side by side
+      std::stable_sort(nodes.begin() + first, nodes.end(), [&](int32_t x, int32_t y) {
+        x &= 0x7fffffff;
+        y &= 0x7fffffff;
+        return h.slot_ptr[x + 1] - h.slot_ptr[x] > h.slot_ptr[y + 1] - h.slot_ptr[y];
+      });
+      if (nodes.size() - first > 0xffffu) return;
+      for (size_t i = first; i < nodes.size(); ++i) at[nodes[i] & 0x7fffffff] = static_cast<int32_t>(i) - first;
+      for (int e = b * chunk; e < e1; ++e)
+        ends[e] = static_cast<uint32_t>(at[h.conn[2 * e]]) | (static_cast<uint32_t>(at[h.conn[2 * e + 1]]) << 16);
+      ptr[b + 1] = static_cast<int32_t>(nodes.size());
+      cap = std::max(cap, ptr[b + 1] - ptr[b]);
+    }
+    const int threads = std::min(most, (std::max(std::min(chunk, most), cap) + 31) / 32 * 32);
+    size_t smem = 0;
+    local.kernel = kernels.local[per_sm - 1];
+    for (int recs = 1; recs >= -1; --recs) {
+      if (recs < 0) return;
+      smem = LocalShape<T>::bytes(cap, recs ? chunk : 0, h.G);
+      local.plan.recs = recs;
+      if (smem <= 232448 && resident_blocks(local.kernel, threads, smem) * sms >= blocks) break;
+    }
+    upload(local_ptr, ptr);
+    upload(local_nodes, nodes);
+    upload(local_ends, ends);
+    local.plan.chunk = chunk;
+    local.plan.cap = cap;
+    local.plan.node_ptr = local_ptr.as<int32_t>();
+    local.plan.nodes = local_nodes.as<int32_t>();
+    local.plan.ends = local_ends.as<uint32_t>();
+    local.blocks = blocks;
+    local.threads = threads;
+    local.smem = smem;
+    ef.alloc(static_cast<size_t>(E) * 24 * sizeof(T));  // two sets of end-force slots
+    DL_CUDA(cudaMemset(ef.p, 0, ef.bytes));
+    m.ef = ef.as<T>();
+  }
+
+  // The records the step kernels read (ElemRecIx, NodeRecIx), from the host model.
+  void upload_records() {
+    const HostLattice &h = *host;
+    const int N = h.N, E = h.E, G = h.G;
+    auto ints = [](T *p, int a, int b, int c, int d) {
+      const int32_t v[4] = {a, b, c, d};
+      std::memcpy(p, v, sizeof v);
+    };
+    if (h.nen == 2) {
+      using Ix = ElemRecIx<T>;
+      const int nv = Ix::vecs(G);
+      std::vector<T> r(static_cast<size_t>(tiles32(E)) * nv * Vec16<T>::n, T(0));
+      for (int e = 0; e < E; ++e) {
+        auto at = [&](int s) { return r.data() + rec_ix<T>(nv, e, s); };
+        ints(at(Ix::ints), h.conn[2 * e], h.conn[2 * e + 1], h.eslot[2 * e], h.eslot[2 * e + 1]);
+        for (int a = 0; a < 2; ++a)
+          for (int k = 0; k < 4; ++k) *at(Ix::qN + 4 * a + k) = T(h.qN[(static_cast<size_t>(a) * E + e) * 4 + k]);
+        for (int k = 0; k < 6; ++k) *at(Ix::C + k) = T(h.C[static_cast<size_t>(k) * E + e]);
+        for (int k = 0; k < 2; ++k) *at(Ix::ec + k) = T(h.ec[static_cast<size_t>(k) * E + e]);
+        for (int k = 0; k < 3; ++k) *at(Ix::k0 + k) = T(h.k0[static_cast<size_t>(k) * E + e]);
+        *at(Ix::L0) = T(1.0 / h.invL0[e]);
+        std::memcpy(at(Ix::invL0), &h.invL0[e], sizeof(double));
+        for (int g = 0; g < G; ++g)
+          for (int k = 0; k < 3; ++k) *at(Ix::g0 + 3 * g + k) = T(h.g0[(static_cast<size_t>(g) * 3 + k) * E + e]);
+      }
+      upload(erec, r);
+      m.erec = erec.as<typename Vec16<T>::type>();
+    }
+    using Nx = NodeRecIx<T>;
+    std::vector<T> r(static_cast<size_t>(tiles32(N)) * Nx::vecs * Vec16<T>::n, T(0));
+    for (int n = 0; n < N; ++n) {
+      auto at = [&](int s) { return r.data() + rec_ix<T>(Nx::vecs, n, s); };
+      int first = h.bc_ptr[n], held = 0;
+      bool zero = true;
+      for (int b = first; b < h.bc_ptr[n + 1]; ++b) {
+        zero = zero && h.bc[b].kind == BCD_DIRICHLET && h.bc[b].scale < 0 && h.bc[b].factor == 0.0;
+        held |= 1 << h.bc[b].dof;
+      }
+      if (zero) first = -1 - held;
+      ints(at(Nx::ints), h.slot_ptr[n], h.slot_ptr[n + 1], first, h.bc_ptr[n + 1]);
+      for (int k = 0; k < 4; ++k) *at(Nx::P + k) = T(h.iframe[static_cast<size_t>(n) * 4 + k]);
+      const double im = 1.0 / h.mass[n];
+      std::memcpy(at(Nx::imass), &im, sizeof im);
+      for (int k = 0; k < 3; ++k) {
+        *at(Nx::D + k) = T(h.idiag[static_cast<size_t>(n) * 4 + k]);
+        *at(Nx::Dinv + k) = T(1.0 / h.idiag[static_cast<size_t>(n) * 4 + k]);
+      }
+    }
+    upload(nrec, r);
+    m.nrec = nrec.as<typename Vec16<T>::type>();
   }
 
   ~Engine() override {
@@ -721,7 +854,7 @@ struct Engine final : EngineBase {
       SampleSpec smp = sample_spec();
       auto enqueue = [&]() {
         if (m.lat_energy) DL_CUDA(cudaMemsetAsync(m.lat_energy, 0, lat_energy.bytes, stream));
-        cudaError_t e = launch_steps<T>(kernels, m, smp, c, exec_mode, barrier.as<GridBarrier>(), stream);
+        cudaError_t e = launch_steps<T>(kernels, m, smp, c, exec_mode, barrier.as<GridBarrier>(), local, stream);
         if (e != cudaSuccess) throw CudaError(std::string("step launch: ") + cudaGetErrorString(e));
         if (has_neumann) {
           e = launch_finish_wext(wstep.as<double>(), n, wext_dev.as<double>(), smp, step, n_samples, c.last_energy,
@@ -778,12 +911,11 @@ struct Engine final : EngineBase {
     if (integ.kind != DL_INTEG_MILNE) {
       mi_pos.alloc(static_cast<size_t>(N) * sizeof(double4));
       mi_rot.alloc(static_cast<size_t>(N) * sizeof(double4));
-      mi_vel.alloc(static_cast<size_t>(N) * 6 * sizeof(double));
+      mi_vel.alloc(vel.bytes);
       if (h.plastic) {
         const size_t NG = static_cast<size_t>(E) * G;
-        mi_ep.alloc(NG * 6 * sizeof(T));
-        mi_al.alloc(NG * nhA * sizeof(T));
-        mi_epsc.alloc(NG * 6 * sizeof(T));
+        mi_hist.alloc(hist.bytes);
+        mi_epsc.alloc(epsc.bytes);
         mi_ediss.alloc(NG * sizeof(double));
       }
       mi_ctl.alloc(sizeof(MilneCtl));
@@ -810,8 +942,7 @@ struct Engine final : EngineBase {
     md.pos_pre = mi_pos.as<double4>();
     md.rot_pre = mi_rot.as<double4>();
     md.vel_pre = mi_vel.as<double>();
-    md.ep_new = mi_ep.as<T>();
-    md.alpha_new = mi_al.as<T>();
+    md.hist_new = mi_hist.as<T>();
     md.epsc_new = mi_epsc.as<T>();
     md.ediss_new = mi_ediss.as<double>();
     md.ctl = mi_ctl.as<MilneCtl>();
@@ -1040,13 +1171,13 @@ struct Engine final : EngineBase {
     const int N = h.N, E = h.E, G = h.G;
     const int nhA = std::max(1, h.nh);
     const size_t NG = static_cast<size_t>(E) * G;
-    const size_t b_pos = static_cast<size_t>(N) * sizeof(double4), b_vel = static_cast<size_t>(N) * 6 * sizeof(double);
-    const size_t b_ep = h.plastic ? NG * 6 * sizeof(T) : 0, b_al = h.plastic ? NG * nhA * sizeof(T) : 0;
+    const size_t b_pos = static_cast<size_t>(N) * sizeof(double4), b_vel = vel.bytes;
+    const size_t b_hist = h.plastic ? hist.bytes : 0, b_epsc = h.plastic ? epsc.bytes : 0;
     const size_t b_ediss = h.plastic ? NG * sizeof(double) : 0;
     // full tape when it fits the memory budget: every step's state is kept
     // during the forward run and nothing is recomputed; otherwise checkpoints
     // every K steps and one recomputation per segment
-    const size_t slot_bytes = 2 * b_pos + b_vel + 2 * b_ep + b_al;
+    const size_t slot_bytes = 2 * b_pos + b_vel + b_hist + b_epsc;
     size_t free_b = 0, total_b = 0;
     DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t budget = tape_budget < 0 ? free_b / 2 : static_cast<size_t>(tape_budget);
@@ -1064,9 +1195,8 @@ struct Engine final : EngineBase {
     ensure_pool(ck_rot, (C + 1) * b_pos);
     ensure_pool(ck_vel, (C + 1) * b_vel);
     if (h.plastic) {
-      ensure_pool(ck_ep, (C + 1) * b_ep);
-      ensure_pool(ck_al, (C + 1) * b_al);
-      ensure_pool(ck_epsc, (C + 1) * b_ep);
+      ensure_pool(ck_hist, (C + 1) * b_hist);
+      ensure_pool(ck_epsc, (C + 1) * b_epsc);
       ensure_pool(ck_ediss, (C + 1) * b_ediss);
     }
     auto d2d = [&](void *dst, const void *src, size_t n) {
@@ -1078,9 +1208,8 @@ struct Engine final : EngineBase {
       d2d(at(ck_rot, c * b_pos), rot.p, b_pos);
       d2d(at(ck_vel, c * b_vel), vel.p, b_vel);
       if (h.plastic) {
-        d2d(at(ck_ep, c * b_ep), ep.p, b_ep);
-        d2d(at(ck_al, c * b_al), alpha.p, b_al);
-        d2d(at(ck_epsc, c * b_ep), epsc.p, b_ep);
+        d2d(at(ck_hist, c * b_hist), hist.p, b_hist);
+        d2d(at(ck_epsc, c * b_epsc), epsc.p, b_epsc);
         d2d(at(ck_ediss, c * b_ediss), ediss.p, b_ediss);
       }
     };
@@ -1089,9 +1218,8 @@ struct Engine final : EngineBase {
       d2d(rot.p, at(ck_rot, c * b_pos), b_pos);
       d2d(vel.p, at(ck_vel, c * b_vel), b_vel);
       if (h.plastic) {
-        d2d(ep.p, at(ck_ep, c * b_ep), b_ep);
-        d2d(alpha.p, at(ck_al, c * b_al), b_al);
-        d2d(epsc.p, at(ck_epsc, c * b_ep), b_ep);
+        d2d(hist.p, at(ck_hist, c * b_hist), b_hist);
+        d2d(epsc.p, at(ck_epsc, c * b_epsc), b_epsc);
         d2d(ediss.p, at(ck_ediss, c * b_ediss), b_ediss);
       }
     };
@@ -1142,8 +1270,7 @@ struct Engine final : EngineBase {
       mm.tp_pos = tb.pos.as<double4>();
       mm.tp_rot = tb.rot.as<double4>();
       mm.tp_vel = tb.vel.as<double>();
-      mm.tp_ep = h.plastic ? tb.ep.as<T>() : nullptr;
-      mm.tp_al = h.plastic ? tb.al.as<T>() : nullptr;
+      mm.tp_hist = h.plastic ? tb.hist.as<T>() : nullptr;
       mm.tp_epsc = h.plastic ? tb.epsc.as<T>() : nullptr;
       mm.tp_step0 = step0;
     };
@@ -1152,16 +1279,15 @@ struct Engine final : EngineBase {
       m.tp_pos = nullptr;
       m.tp_rot = nullptr;
       m.tp_vel = nullptr;
-      m.tp_ep = m.tp_al = m.tp_epsc = nullptr;
+      m.tp_hist = m.tp_epsc = nullptr;
     };
     auto tape_slot0 = [&](StateTape &tb) {  // current state into slot 0
       d2d(tb.pos.p, pos.p, b_pos);
       d2d(tb.rot.p, rot.p, b_pos);
       d2d(tb.vel.p, vel.p, b_vel);
       if (h.plastic) {
-        d2d(tb.ep.p, ep.p, b_ep);
-        d2d(tb.al.p, alpha.p, b_al);
-        d2d(tb.epsc.p, epsc.p, b_ep);
+        d2d(tb.hist.p, hist.p, b_hist);
+        d2d(tb.epsc.p, epsc.p, b_epsc);
       }
     };
     // tape of one segment (K + 1 slots; the whole run when full); a second
@@ -1172,9 +1298,8 @@ struct Engine final : EngineBase {
       ensure_pool(tape[b].rot, static_cast<size_t>(K + 1) * b_pos);
       ensure_pool(tape[b].vel, static_cast<size_t>(K + 1) * b_vel);
       if (h.plastic) {
-        ensure_pool(tape[b].ep, static_cast<size_t>(K + 1) * b_ep);
-        ensure_pool(tape[b].al, static_cast<size_t>(K + 1) * b_al);
-        ensure_pool(tape[b].epsc, static_cast<size_t>(K + 1) * b_ep);
+        ensure_pool(tape[b].hist, static_cast<size_t>(K + 1) * b_hist);
+        ensure_pool(tape[b].epsc, static_cast<size_t>(K + 1) * b_epsc);
       }
     }
     for (int64_t c = 0; c < C; ++c) {
@@ -1513,14 +1638,12 @@ struct Engine final : EngineBase {
     const int E = h.E, G = h.G, nh = h.nh;
     DL_CUDA(cudaStreamSynchronize(stream));
     const size_t NG = static_cast<size_t>(E) * G;
-    std::vector<T> a, b;
+    std::vector<T> a;
     std::vector<double> d;
     if (h.plastic) {
-      a.resize(NG * 6);
-      b.resize(NG * std::max(1, nh));
+      a.resize(hist.bytes / sizeof(T));
       d.resize(NG);
-      DL_CUDA(cudaMemcpy(a.data(), ep.p, a.size() * sizeof(T), cudaMemcpyDeviceToHost));
-      DL_CUDA(cudaMemcpy(b.data(), alpha.p, b.size() * sizeof(T), cudaMemcpyDeviceToHost));
+      DL_CUDA(cudaMemcpy(a.data(), hist.p, hist.bytes, cudaMemcpyDeviceToHost));
       DL_CUDA(cudaMemcpy(d.data(), ediss.p, d.size() * sizeof(double), cudaMemcpyDeviceToHost));
     }
     for (int e = 0; e < E; ++e) {
@@ -1528,9 +1651,9 @@ struct Engine final : EngineBase {
       for (int g = 0; g < G; ++g) {
         const size_t o = static_cast<size_t>(e) * G + g;
         for (int k = 0; k < 6; ++k)
-          if (epo) epo[o * 6 + k] = h.plastic ? double(a[(static_cast<size_t>(g) * 6 + k) * E + ei]) : 0.0;
+          if (epo) epo[o * 6 + k] = h.plastic ? double(a[hist_ix<T>(G, m.hs, ei, g, k)]) : 0.0;
         for (int k = 0; k < 7; ++k)
-          if (hpo) hpo[o * 7 + k] = (h.plastic && k < nh) ? double(b[(static_cast<size_t>(g) * nh + k) * E + ei]) : 0.0;
+          if (hpo) hpo[o * 7 + k] = (h.plastic && k < nh) ? double(a[hist_ix<T>(G, m.hs, ei, g, 6 + k)]) : 0.0;
         if (edo) edo[o] = h.plastic ? d[static_cast<size_t>(g) * E + ei] : 0.0;
       }
     }

@@ -25,6 +25,10 @@ struct KernelSet {
   const void *node_x = nullptr;
   const void *internal_force = nullptr;
   const void *gather = nullptr;
+  // one grid barrier per step, node copies in shared memory (local.cuh): for at
+  // most one block per SM, and for two
+  const void *local[2] = {nullptr, nullptr};
+  int local_threads = 256;      // most threads of its blocks (LocalThreads)
   const void *milne = nullptr;  // MilneDevice predictor-corrector (milne.cuh)
   int full_threads = 256;    // threads of a full persistent block (PersistShape) ...
   int full_threads_x = 256;  // ... and of the extended variant
@@ -42,6 +46,14 @@ struct KernelSet {
 // more SMs, so each warp gets more of its SM's issue slots.
 int threads_for(int work);
 
+// Models of at most this many elements, nodes and pairs run in one block, whose
+// own barrier then replaces the grid's: two grid barriers are 3.5 us of a step.
+// FP64 rods, us per step, several blocks against one: 33 nodes 8.7 / 5.3, 128
+// nodes 10.2 / 5.8, 249 nodes (two items per thread) 9.3 / 8.6; an elastoplastic
+// 2^3 BCC lattice (163 nodes, 128 elements) 14.0 / 9.6.  Above that the one SM's
+// FP64 units and the items each thread walks cost what the barriers did.
+constexpr int kSoloWork = 256;
+
 // Entry points of the two reverse-step kernels (adjoint_kernels.cuh).
 struct AdjKernels {
   const void *node = nullptr;
@@ -58,9 +70,19 @@ KernelSet aot_kernels(bool plastic);
 int cooperative_blocks(const void *kernel, int threads);
 // fills ks.persist_blocks and ks.persist_cap
 void set_persistent_caps(KernelSet &ks);
+// Launch shape of the one-barrier step kernel for a model (blocks = 0: the model
+// does not fit it).
+struct LocalLaunch {
+  const void *kernel = nullptr;
+  int blocks = 0, threads = 0;
+  size_t smem = 0;
+  LocalPlan plan;
+};
+// Blocks of `threads` threads and `smem` bytes that are resident on an SM (0 if none).
+int resident_blocks(const void *kernel, int threads, size_t smem);
 template <class T>
 cudaError_t launch_steps(const KernelSet &ks, const DevModel<T> &m, const SampleSpec &smp, const StepCtx &c,
-                         int mode, GridBarrier *bar, cudaStream_t s);
+                         int mode, GridBarrier *bar, const LocalLaunch &local, cudaStream_t s);
 template <class T>
 cudaError_t launch_internal_force(const KernelSet &ks, const DevModel<T> &m, double *fint, cudaStream_t s);
 // One persistent launch of the predictor-corrector over c.nsteps accepted

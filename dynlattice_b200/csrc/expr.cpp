@@ -250,6 +250,21 @@ struct Builder {
     return id;
   }
 
+  // a^k: whole exponents from 2 to 8 as products (a general pow costs a hundred
+  // instructions and more, and a yield function asks for one at every point)
+  int power(int a, int k) {
+    if (code[k].op == XO_CONST && code[k].k >= 2.0 && code[k].k <= 8.0 && code[k].k == std::floor(code[k].k)) {
+      const int e = static_cast<int>(code[k].k);
+      const int sq = emit(XO_SQUARE, a);
+      if (e <= 3) return e == 2 ? sq : emit(XO_MUL, sq, a);
+      const int q4 = emit(XO_SQUARE, sq);
+      if (e == 8) return emit(XO_SQUARE, q4);
+      const int rest = e == 4 ? -1 : (e == 5 ? a : (e == 6 ? sq : emit(XO_MUL, sq, a)));
+      return rest < 0 ? q4 : emit(XO_MUL, q4, rest);
+    }
+    return emit(XO_POW, a, k);
+  }
+
   int build(const ExprNode *n) {
     switch (n->kind) {
       case ExprNode::NUM: return emit(XO_CONST, -1, -1, -1, n->num);
@@ -262,8 +277,7 @@ struct Builder {
         int a = build(n->kids[0].get());
         int b = build(n->kids[1].get());
         int op = binOps().at(n->op);
-        if (op == XO_POW && code[b].op == XO_CONST && code[b].k == 2.0) return emit(XO_SQUARE, a);
-        return emit(op, a, b);
+        return op == XO_POW ? power(a, b) : emit(op, a, b);
       }
       case ExprNode::CALL: {
         const std::string &f = n->op;
@@ -279,7 +293,8 @@ struct Builder {
         }
         if (f == "pow") {
           if (n->kids.size() != 2) throw std::runtime_error("pow() takes two arguments");
-          return emit(XO_POW, build(n->kids[0].get()), build(n->kids[1].get()));
+          const int a = build(n->kids[0].get());
+          return power(a, build(n->kids[1].get()));
         }
         if (f == "min" || f == "max") {
           if (n->kids.empty()) throw std::runtime_error(f + "() needs arguments");
@@ -411,7 +426,13 @@ ExprProgram compileExprs(const std::vector<ExprPtr> &exprs) {
 
 namespace {
 
-std::string emitSsa(const Builder &b, const std::vector<int> &live, bool fp32, std::vector<std::string> &names) {
+// `given`: names of values computed elsewhere (not emitted); `recip`: of their
+// reciprocals, for divisions.
+// With `given`, multiply-adds are written out (mul_rn, fma_rn of the step kernels):
+// the kernels that share the code must round alike, whatever the compiler would
+// contract in each.
+std::string emitSsa(const Builder &b, const std::vector<int> &live, bool fp32, std::vector<std::string> &names,
+                    const std::vector<std::string> *given = nullptr, const std::vector<std::string> *recip = nullptr) {
   const char *T = fp32 ? "float" : "double";
   auto fn = [&](const char *d) { return fp32 ? std::string(d) + "f" : std::string(d); };
   std::string out;
@@ -420,21 +441,52 @@ std::string emitSsa(const Builder &b, const std::vector<int> &live, bool fp32, s
   for (size_t i = 0; i < b.code.size(); ++i) {
     if (!live[i]) continue;
     const SsaInst &in = b.code[i];
+    if (given && !(*given)[i].empty()) {
+      names[i] = (*given)[i];
+      continue;
+    }
     std::string nm = "r" + std::to_string(i);
     names[i] = nm;
     auto A = [&](int r) { return names[r]; };
     std::string e;
+    // the factors of a value that is a product
+    auto product = [&](int r, std::string &x, std::string &y) {
+      const SsaInst &p = b.code[r];
+      if (!given || !(*given)[r].empty()) return false;
+      if (p.op == XO_SQUARE) x = y = A(p.a);
+      else if (p.op == XO_MUL) x = A(p.a), y = A(p.b);
+      else if (p.op == XO_DIV && !(*recip)[p.b].empty()) x = A(p.a), y = (*recip)[p.b];
+      else return false;
+      return true;
+    };
+    std::string px, py;
+    auto mul = [&](const std::string &x, const std::string &y) {
+      return given ? "mul_rn(" + x + ", " + y + ")" : x + " * " + y;
+    };
+    auto fma = [&](const std::string &x, const std::string &y, const std::string &z) {
+      return "fma_rn(" + x + ", " + y + ", " + z + ")";
+    };
     switch (in.op) {
       case XO_CONST:
         std::snprintf(buf, sizeof buf, "%s(%.17g)", T, in.k);
         e = buf;
         break;
       case XO_ARG: e = "a[" + std::to_string(in.a) + "]"; break;
-      case XO_ADD: e = A(in.a) + " + " + A(in.b); break;
-      case XO_SUB: e = A(in.a) + " - " + A(in.b); break;
-      case XO_MUL: e = A(in.a) + " * " + A(in.b); break;
-      case XO_DIV: e = A(in.a) + " / " + A(in.b); break;
-      case XO_SQUARE: e = A(in.a) + " * " + A(in.a); break;
+      case XO_ADD:
+        if (product(in.b, px, py)) e = fma(px, py, A(in.a));
+        else if (product(in.a, px, py)) e = fma(px, py, A(in.b));
+        else e = A(in.a) + " + " + A(in.b);
+        break;
+      case XO_SUB:
+        if (product(in.b, px, py)) e = fma("-" + px, py, A(in.a));
+        else if (product(in.a, px, py)) e = fma(px, py, "-" + A(in.b));
+        else e = A(in.a) + " - " + A(in.b);
+        break;
+      case XO_MUL: e = mul(A(in.a), A(in.b)); break;
+      case XO_DIV:
+        e = recip && !(*recip)[in.b].empty() ? mul(A(in.a), (*recip)[in.b]) : A(in.a) + " / " + A(in.b);
+        break;
+      case XO_SQUARE: e = mul(A(in.a), A(in.a)); break;
       case XO_POW: e = fn("pow") + "(" + A(in.a) + ", " + A(in.b) + ")"; break;
       case XO_NEG: e = "-" + A(in.a); break;
       case XO_ABS: e = fn("fabs") + "(" + A(in.a) + ")"; break;
@@ -487,30 +539,102 @@ std::vector<int> liveSet(const Builder &b, const std::vector<int> &outs) {
 
 }  // namespace
 
+namespace {
+
+// Code of several expressions in two parts.  Their values that depend on the
+// element's own variables only (arguments `own_from` and up: radius, area) are
+// the same at every point and iteration: `prep` stores those that the rest
+// reads, or their reciprocals where the rest divides by them, to inv[0 .. count);
+// `body` is the rest, with names[i] the value of outs[i].
+struct TwoPart {
+  std::string prep, body;
+  std::vector<std::string> names;
+  int count = 0;
+};
+TwoPart emitTwoPart(const std::vector<ExprPtr> &exprs, int own_from, bool fp32) {
+  const std::string T = fp32 ? "float" : "double";
+  Builder b;
+  std::vector<int> outs;
+  for (auto &e : exprs) outs.push_back(b.build(e.get()));
+  const std::vector<int> live = liveSet(b, outs);
+  const size_t n = b.code.size();
+  std::vector<char> own(n, 0), constant(n, 0);
+  for (size_t i = 0; i < n; ++i) {
+    const SsaInst &in = b.code[i];
+    if (in.op == XO_CONST) {
+      own[i] = constant[i] = 1;
+    } else if (in.op == XO_ARG) {
+      own[i] = in.a >= own_from;
+    } else {
+      own[i] = 1;
+      for (int r : {in.a, in.b, in.c}) own[i] = own[i] && (r < 0 || own[r]);
+    }
+  }
+  std::vector<std::string> given(n), recip(n);
+  std::vector<int> slots, recips;
+  TwoPart out;
+  auto slot = [&] { return "inv[" + std::to_string(out.count++) + "]"; };
+  auto read = [&](int r) {
+    if (r < 0 || !own[r] || constant[r] || !given[r].empty()) return;
+    given[r] = slot();
+    slots.push_back(r);
+  };
+  for (size_t i = 0; i < n; ++i) {
+    const SsaInst &in = b.code[i];
+    if (!live[i] || own[i] || in.op == XO_ARG) continue;
+    if (in.op == XO_DIV && own[in.b] && !constant[in.b]) {
+      read(in.a);
+      if (recip[in.b].empty()) {
+        recip[in.b] = slot();
+        recips.push_back(in.b);
+      }
+      continue;
+    }
+    for (int r : {in.a, in.b, in.c}) read(r);
+  }
+  for (int o : outs) read(o);
+  std::vector<int> all = slots;
+  all.insert(all.end(), recips.begin(), recips.end());
+  std::vector<std::string> nm;
+  if (!all.empty()) out.prep = emitSsa(b, liveSet(b, all), fp32, nm);
+  for (int r : slots) out.prep += "    " + given[r] + " = " + nm[r] + ";\n";
+  for (int r : recips) out.prep += "    " + recip[r] + " = " + T + "(1) / " + nm[r] + ";\n";
+  std::vector<int> rest(n, 0), stack = outs;
+  while (!stack.empty()) {
+    const int r = stack.back();
+    stack.pop_back();
+    if (r < 0 || rest[r]) continue;
+    rest[r] = 1;
+    const SsaInst &in = b.code[r];
+    if (in.op == XO_CONST || in.op == XO_ARG || !given[r].empty()) continue;
+    stack.push_back(in.a);
+    if (!(in.op == XO_DIV && !recip[in.b].empty())) stack.push_back(in.b);
+    stack.push_back(in.c);
+  }
+  std::vector<std::string> names;
+  out.body = emitSsa(b, rest, fp32, names, &given, &recip);
+  for (int o : outs) out.names.push_back(names[o]);
+  return out;
+}
+
+}  // namespace
+
 std::string emitYieldPolicy(const ExprPtr &f, const std::vector<ExprPtr> &grads, bool fp32) {
-  const char *T = fp32 ? "float" : "double";
+  const std::string T = fp32 ? "float" : "double";
+  const int nh = static_cast<int>(grads.size()) - 6;
+  const TwoPart tf = emitTwoPart({f}, 6 + nh, fp32), tg = emitTwoPart(grads, 6 + nh, fp32);
+  const std::string dev = "  __device__ static __forceinline__ ", arg = "const " + T + " *__restrict__ a";
   std::string src = "struct YieldJit {\n  static constexpr bool kPlastic = true;\n  static constexpr int kNh = " +
-                    std::to_string(static_cast<int>(grads.size()) - 6) + ";\n  static constexpr int kMinBlocks = 2;\n";
-  {
-    Builder b;
-    int o = b.build(f.get());
-    std::vector<std::string> names;
-    std::string body = emitSsa(b, liveSet(b, {o}), fp32, names);
-    src += "  __device__ static __forceinline__ " + std::string(T) + " f(const DevModel<" + T + "> &, const " + T +
-           " *__restrict__ a, " + T + " *) {\n" + body + "    return " + names[o] + ";\n  }\n";
-  }
-  {
-    Builder b;
-    std::vector<int> outs;
-    for (auto &g : grads) outs.push_back(b.build(g.get()));
-    std::vector<std::string> names;
-    std::string body = emitSsa(b, liveSet(b, outs), fp32, names);
-    src += "  __device__ static __forceinline__ void grad(const DevModel<" + std::string(T) + "> &, const " + T +
-           " *__restrict__ a, " + T + " *g, " + T + " *) {\n" + body;
-    for (size_t k = 0; k < outs.size(); ++k) src += "    g[" + std::to_string(k) + "] = " + names[outs[k]] + ";\n";
-    src += "  }\n";
-  }
-  src += "};\n";
+                    std::to_string(nh) + ";\n  static constexpr int kMinBlocks = 2;\n  static constexpr int kRegs = 1;\n";
+  src += "  static constexpr int kInv = " + std::to_string(tf.count) + ", kGradInv = " + std::to_string(tg.count) + ";\n";
+  src += dev + "void prep(" + arg + ", " + T + " *inv) {\n" + tf.prep + "  }\n";
+  src += dev + "void prep_grad(" + arg + ", " + T + " *inv) {\n" + tg.prep + "  }\n";
+  src += dev + T + " f(const DevModel<" + T + "> &, " + arg + ", const " + T + " *inv, " + T + " *) {\n" + tf.body +
+         "    return " + tf.names[0] + ";\n  }\n";
+  src += dev + "void grad(const DevModel<" + T + "> &, " + arg + ", const " + T + " *inv, " + T + " *g, " + T + " *) {\n" +
+         tg.body;
+  for (size_t k = 0; k < tg.names.size(); ++k) src += "    g[" + std::to_string(k) + "] = " + tg.names[k] + ";\n";
+  src += "  }\n};\n";
   return src;
 }
 

@@ -20,7 +20,7 @@ namespace dl {
 
 namespace {
 
-constexpr int kNames = 10;
+constexpr int kNames = 12;
 
 struct Entry {
   cudaLibrary_t lib = nullptr;
@@ -165,7 +165,7 @@ std::map<std::string, std::pair<cudaLibrary_t, AdjKernels>> g_adj_cache;
 bool jit_compile(const std::string &policy_source, bool fp32, std::vector<char> *cubin,
                  std::vector<std::string> *lowered, std::string *log) {
   const char *T = fp32 ? "float" : "double";
-  const std::string src = "#include \"milne.cuh\"\nnamespace dl {\n" + policy_source + "}\n";
+  const std::string src = "#include \"milne.cuh\"\n#include \"local.cuh\"\nnamespace dl {\n" + policy_source + "}\n";
   const std::vector<std::string> names = {
       std::string("&dl::k_persistent<") + T + ", dl::YieldJit, false>",
       std::string("&dl::k_element<") + T + ", dl::YieldJit, false>",
@@ -176,7 +176,9 @@ bool jit_compile(const std::string &policy_source, bool fp32, std::vector<char> 
       std::string("&dl::k_element<") + T + ", dl::YieldJit, true>",
       std::string("&dl::k_node<") + T + ", true>",
       std::string("&dl::k_milne<") + T + ", dl::YieldJit>",
-      std::string("&dl::k_persistent<") + T + ", dl::YieldJit, false, true>"};
+      std::string("&dl::k_persistent<") + T + ", dl::YieldJit, false, true>",
+      std::string("&dl::k_local<") + T + ", dl::YieldJit, 1>",
+      std::string("&dl::k_local<") + T + ", dl::YieldJit, 2>"};
   return compile_generic(src, names, fp32, "step", cubin, lowered, log);
 }
 
@@ -255,6 +257,9 @@ const KernelSet *jit_kernels(const std::string &policy_source, bool fp32, std::s
   e->ks.node_x = reinterpret_cast<const void *>(k[7]);
   e->ks.milne = reinterpret_cast<const void *>(k[8]);
   e->ks.persistent1 = reinterpret_cast<const void *>(k[9]);
+  e->ks.local[0] = reinterpret_cast<const void *>(k[10]);
+  e->ks.local[1] = reinterpret_cast<const void *>(k[11]);
+  e->ks.local_threads = fp32 ? 320 : 256;  // LocalThreads<T>
   e->ks.full_threads = fp32 ? 320 : 256;  // PersistShape<T, false>::kThreads
   e->ks.full_threads_x = 256;             // PersistShape<T, true>::kThreads
   set_persistent_caps(e->ks);

@@ -8,6 +8,7 @@
 
 #include "engine.hpp"
 #include "rodkin.cuh"
+#include "local.cuh"
 #include "milne.cuh"
 
 namespace dl {
@@ -67,7 +68,7 @@ __global__ void k_state_out(const double4 *pos, const double4 *rot, const double
       th[n * 3 + 2] = t.z;
     }
     if (v)
-      for (int k = 0; k < 6; ++k) v[n * 6 + k] = vel[k * N + i];
+      for (int k = 0; k < 6; ++k) v[n * 6 + k] = vel[vel_ix(i, k)];
   }
 }
 
@@ -81,7 +82,7 @@ __global__ void k_state_in(double4 *pos, double4 *rot, double *vel, const double
       rot[i] = make_double4(q.w, q.x, q.y, q.z);
     }
     if (v)
-      for (int k = 0; k < 6; ++k) vel[k * N + i] = v[n * 6 + k];
+      for (int k = 0; k < 6; ++k) vel[vel_ix(i, k)] = v[n * 6 + k];
   }
 }
 
@@ -127,6 +128,16 @@ void set_persistent_caps(KernelSet &ks) {
   ks.persist_blocks = ks.persist_cap[3];
 }
 
+int resident_blocks(const void *kernel, int threads, size_t smem) {
+  int occ = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return occ;
+}
+
 int cooperative_blocks(const void *kernel, int threads) {
   int dev = 0, sms = 0, occ = 0;
   cudaGetDevice(&dev);
@@ -151,6 +162,9 @@ static KernelSet aot_set() {
   k.node_x = reinterpret_cast<const void *>(k_node<T, true>);
   k.internal_force = reinterpret_cast<const void *>(k_internal_force<T, Y>);
   k.gather = reinterpret_cast<const void *>(k_gather_force<T>);
+  k.local[0] = reinterpret_cast<const void *>(k_local<T, Y, 1>);
+  k.local[1] = reinterpret_cast<const void *>(k_local<T, Y, 2>);
+  k.local_threads = LocalThreads<T>::value;
   k.milne = reinterpret_cast<const void *>(k_milne<T, Y>);
   k.full_threads = PersistShape<T, false>::kThreads;
   k.full_threads_x = PersistShape<T, true>::kThreads;
@@ -164,26 +178,23 @@ KernelSet aot_kernels(bool plastic) {
   return plastic ? aot_set<T, YieldInterp>() : aot_set<T, ElasticOnly>();
 }
 
-// Models of at most this many elements, nodes and pairs run in one block, whose
-// own barrier then replaces the grid's: two grid barriers are 3.5 us of a step.
-// FP64 rods, us per step, several blocks against one: 33 nodes 8.7 / 5.3, 128
-// nodes 10.2 / 5.8, 249 nodes (two items per thread) 9.3 / 8.6; an elastoplastic
-// 2^3 BCC lattice (163 nodes, 128 elements) 14.0 / 9.6.  Above that the one SM's
-// FP64 units and the items each thread walks cost what the barriers did.
-constexpr int kSoloWork = 256;
-
 template <class T>
 cudaError_t launch_steps(const KernelSet &ks, const DevModel<T> &m, const SampleSpec &smp, const StepCtx &c,
-                         int mode, GridBarrier *bar, cudaStream_t s) {
+                         int mode, GridBarrier *bar, const LocalLaunch &local, cudaStream_t s) {
   if (c.nsteps <= 0) return cudaSuccess;
   // the extended kernels only when the model or the run uses their features
-  const bool ext = m.c_ptr || m.j_ptr || m.n_plates > 0 || m.tp_pos || m.tp_ep || m.grp_hist || m.fint_last ||
+  const bool ext = m.c_ptr || m.j_ptr || m.n_plates > 0 || m.tp_pos || m.tp_hist || m.grp_hist || m.fint_last ||
                    m.br || m.lumped || m.tie_ptr || m.nen > 2;
   DevModel<T> mm = m;
   SampleSpec ss = smp;
   StepCtx cc = c;
   if (mode == EXEC_PERSISTENT || mode == EXEC_GRAPH) {
     GridBarrier *bb = bar;
+    if (local.blocks > 0 && !ext && c.nsteps > 1 && ks.tpb_override <= 0) {
+      LocalPlan pl = local.plan;
+      void *la[] = {&mm, &ss, &cc, &bb, &pl};
+      return cudaLaunchCooperativeKernel(local.kernel, dim3(local.blocks), dim3(local.threads), la, local.smem, s);
+    }
     void *args[] = {&mm, &ss, &cc, &bb};
     // one element or node per thread at most: small models take few blocks,
     // which keeps the grid barriers short
@@ -281,7 +292,7 @@ __global__ void k_elem_table(const DevModel<T> m, int kind, int spatial, double 
         const Q4<T> qg = cvtq<T>(k.L);
         T val[6];
         for (int q = 0; q < 6; ++q) {
-          const T ep = m.plastic ? m.ep[(g * 6 + q) * E + e] : T(0);
+          const T ep = m.plastic ? m.hist[hist_ix<T>(G, m.hs, e, g, q)] : T(0);
           val[q] = kind == 0 ? eps[q] : (kind == 1 ? T(m.C[q * E + e]) * (eps[q] - ep) : ep);
         }
         if (spatial) {
@@ -295,8 +306,9 @@ __global__ void k_elem_table(const DevModel<T> m, int kind, int spatial, double 
       for (int q = 0; q < 6; ++q) out[static_cast<size_t>(e) * 6 + q] = acc[q] * G;
       continue;
     }
-    ElemPre<T> p;
-    elem_pre(m, e, m.pos, m.rot, p);
+    ElemPre<T, ElasticOnly> p;
+    elem_pre(m, e, G, GlobalEnds{m.pos, m.rot}, p);
+    const T il = T(m.invL0[e]);
     const Q4<T> epair = qexp((T(-0.5) * T(c_gxi[G - 1][G - 1])) * p.k.phi);
     double acc[6] = {0, 0, 0, 0, 0, 0};
     for (int g = 0; g < G; ++g) {
@@ -309,10 +321,10 @@ __global__ void k_elem_table(const DevModel<T> m, int kind, int spatial, double 
       }
       T eps[6];
       Q4<T> qg;
-      gp_strain_e(p.k, eg, p.il, g0, k0, eps, &qg);
+      gp_strain_e(p.k, eg, il, g0, k0, eps, &qg);
       T val[6];
       for (int k = 0; k < 6; ++k) {
-        const T ep = m.plastic ? m.ep[(g * 6 + k) * E + e] : T(0);
+        const T ep = m.plastic ? m.hist[hist_ix<T>(G, m.hs, e, g, k)] : T(0);
         val[k] = kind == 0 ? eps[k] : (kind == 1 ? p.Cd[k] * (eps[k] - ep) : ep);
       }
       if (spatial) {
@@ -354,7 +366,8 @@ cudaError_t launch_state_in(double4 *pos, double4 *rot, double *vel, const doubl
 #define DL_INSTANTIATE(T)                                                                              \
   template KernelSet aot_kernels<T>(bool);                                                                 \
   template cudaError_t launch_steps<T>(const KernelSet &, const DevModel<T> &, const SampleSpec &,     \
-                                       const StepCtx &, int, GridBarrier *, cudaStream_t);            \
+                                       const StepCtx &, int, GridBarrier *, const LocalLaunch &,           \
+                                       cudaStream_t);                                                 \
   template cudaError_t launch_internal_force<T>(const KernelSet &, const DevModel<T> &, double *,     \
                                                 cudaStream_t);                                        \
   template cudaError_t launch_milne<T>(const KernelSet &, const DevModel<T> &, const SampleSpec &,     \

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256, Y::kMinBlocks)
   const int gstride = gridDim.x * blockDim.x;
   const int N = m.N, E = m.E, G = m.G;
   const int nh = Y::kNh >= 0 ? Y::kNh : m.nh;
-  const HistOut<T> ho{md.ep_new, md.alpha_new, md.epsc_new, md.ediss_new};
+  const HistOut<T> ho{md.hist_new, md.epsc_new, md.ediss_new};
   double t = md.ctl->t, dt = md.ctl->dt;
   int64_t step = md.ctl->step, rejected = md.ctl->rejected;
   const double inv_rms = 1.0 / sqrt(6.0 * double(N));
@@ -142,11 +142,14 @@ __global__ void __launch_bounds__(256, Y::kMinBlocks)
       if (!m.plastic) return;
       for (int e = gtid; e < E; e += gstride)
         for (int g = 0; g < G; ++g) {
-          for (int k = 0; k < 6; ++k) {
-            m.ep[(g * 6 + k) * E + e] = md.ep_new[(g * 6 + k) * E + e];
-            m.epsc[(g * 6 + k) * E + e] = md.epsc_new[(g * 6 + k) * E + e];
+          for (int k = 0; k < 6 + nh; ++k) {
+            const size_t i = hist_ix<T>(G, m.hs, e, g, k);
+            m.hist[i] = md.hist_new[i];
           }
-          for (int a = 0; a < nh; ++a) m.alpha[(g * nh + a) * E + e] = md.alpha_new[(g * nh + a) * E + e];
+          for (int k = 0; k < 6; ++k) {
+            const size_t i = epsc_ix(G, e, g, k);
+            m.epsc[i] = md.epsc_new[i];
+          }
           m.ediss[g * E + e] = md.ediss_new[g * E + e];
         }
     }
@@ -183,12 +186,12 @@ __global__ void __launch_bounds__(256, Y::kMinBlocks)
     for (int n = gtid; n < N; n += gstride) {
       double v[6];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) v[k] = vel_cur[k * N + n];
+      for (int k = 0; k < 6; ++k) v[k] = vel_cur[vel_ix(n, k)];
       const V3<double> x = ldx(pos_cur + n);
       const Q4<double> R = ldq(rot_cur + n);
       if (acc_prev) {  // the accepted state becomes the current one
 #pragma unroll
-        for (int k = 0; k < 6; ++k) m.vel[k * N + n] = v[k];
+        for (int k = 0; k < 6; ++k) m.vel[vel_ix(n, k)] = v[k];
         m.pos[n] = make_double4(x.x, x.y, x.z, 0.0);
         m.rot[n] = make_double4(R.w, R.x, R.y, R.z);
       }
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(256, Y::kMinBlocks)
       const V3<double> xp = x + dt * V3<double>{v[0], v[1], v[2]};
       const Q4<double> Rp = milne_rotate(m, R, dt * V3<double>{v[3], v[4], v[5]});
 #pragma unroll
-      for (int k = 0; k < 6; ++k) md.vel_pre[k * N + n] = v[k] + dt * a[k];
+      for (int k = 0; k < 6; ++k) md.vel_pre[vel_ix(n, k)] = v[k] + dt * a[k];
       md.pos_pre[n] = make_double4(xp.x, xp.y, xp.z, 0.0);
       md.rot_pre[n] = make_double4(Rp.w, Rp.x, Rp.y, Rp.z);
     }
@@ -231,8 +234,8 @@ __global__ void __launch_bounds__(256, Y::kMinBlocks)
       double v[6], vp[6];
 #pragma unroll
       for (int k = 0; k < 6; ++k) {
-        v[k] = m.vel[k * N + n];
-        vp[k] = md.vel_pre[k * N + n];
+        v[k] = m.vel[vel_ix(n, k)];
+        vp[k] = md.vel_pre[vel_ix(n, k)];
       }
       const V3<double> x = ldx(m.pos + n);
       const Q4<double> R = ldq(m.rot + n), Rp = ldq(md.rot_pre + n);
@@ -274,7 +277,7 @@ __global__ void __launch_bounds__(256, Y::kMinBlocks)
       for (int k = 0; k < 6; ++k) finite = finite && isfinite(vn[k]);
       if (!finite) atomicOr(m.err, 0x2u);
 #pragma unroll
-      for (int k = 0; k < 6; ++k) md.vel_pre[k * N + n] = vn[k];
+      for (int k = 0; k < 6; ++k) md.vel_pre[vel_ix(n, k)] = vn[k];
       md.pos_pre[n] = make_double4(xn.x, xn.y, xn.z, 0.0);
       md.rot_pre[n] = make_double4(Rn.w, Rn.x, Rn.y, Rn.z);
       if (sidx >= 0 && smp.n_watch > 0) {
@@ -362,7 +365,7 @@ __global__ void __launch_bounds__(256, Y::kMinBlocks)
     commit_history();
     for (int n = gtid; n < N; n += gstride) {
 #pragma unroll
-      for (int k = 0; k < 6; ++k) m.vel[k * N + n] = md.vel_pre[k * N + n];
+      for (int k = 0; k < 6; ++k) m.vel[vel_ix(n, k)] = md.vel_pre[vel_ix(n, k)];
       m.pos[n] = md.pos_pre[n];
       m.rot[n] = md.rot_pre[n];
     }

@@ -51,13 +51,45 @@ template <class T>
 DL_HD V3<T> operator*(T s, V3<T> a) {
   return V3<T>{s * a.x, s * a.y, s * a.z};
 }
+// a b + c and a b, rounded as written on the device (one rounding each), so that
+// every kernel that shares a formula gets the same bits; the host evaluates them
+// plainly.
+DL_HD float fma_rn(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  return __fmaf_rn(a, b, c);
+#else
+  return a * b + c;
+#endif
+}
+DL_HD double fma_rn(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+  return __fma_rn(a, b, c);
+#else
+  return a * b + c;
+#endif
+}
+DL_HD float mul_rn(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+DL_HD double mul_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
 template <class T>
 DL_HD T dot(V3<T> a, V3<T> b) {
-  return a.x * b.x + a.y * b.y + a.z * b.z;
+  return fma_rn(a.z, b.z, fma_rn(a.y, b.y, mul_rn(a.x, b.x)));
 }
 template <class T>
 DL_HD V3<T> cross(V3<T> a, V3<T> b) {
-  return V3<T>{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+  return V3<T>{fma_rn(a.y, b.z, -mul_rn(a.z, b.y)), fma_rn(a.z, b.x, -mul_rn(a.x, b.z)),
+               fma_rn(a.x, b.y, -mul_rn(a.y, b.x))};
 }
 template <class T, class U>
 DL_HD V3<T> cvt(V3<U> a) {
@@ -70,10 +102,10 @@ DL_HD Q4<T> cvtq(Q4<U> a) {
 
 template <class T>
 DL_HD Q4<T> qmul(Q4<T> a, Q4<T> b) {
-  return Q4<T>{a.w * b.w - a.x * b.x - a.y * b.y - a.z * b.z,
-               a.w * b.x + a.x * b.w + a.y * b.z - a.z * b.y,
-               a.w * b.y - a.x * b.z + a.y * b.w + a.z * b.x,
-               a.w * b.z + a.x * b.y - a.y * b.x + a.z * b.w};
+  return Q4<T>{fma_rn(-a.z, b.z, fma_rn(-a.y, b.y, fma_rn(-a.x, b.x, mul_rn(a.w, b.w)))),
+               fma_rn(-a.z, b.y, fma_rn(a.y, b.z, fma_rn(a.x, b.w, mul_rn(a.w, b.x)))),
+               fma_rn(a.z, b.x, fma_rn(a.y, b.w, fma_rn(-a.x, b.z, mul_rn(a.w, b.y)))),
+               fma_rn(a.z, b.w, fma_rn(-a.y, b.x, fma_rn(a.x, b.y, mul_rn(a.w, b.z))))};
 }
 template <class T>
 DL_HD Q4<T> qconj(Q4<T> a) {
@@ -86,7 +118,7 @@ DL_HD V3<T> qrot_delta(Q4<T> q, V3<T> v) {
   V3<T> u{q.x, q.y, q.z};
   V3<T> t = cross(u, v);
   V3<T> tt = cross(u, t);
-  return V3<T>{T(2) * (q.w * t.x + tt.x), T(2) * (q.w * t.y + tt.y), T(2) * (q.w * t.z + tt.z)};
+  return V3<T>{T(2) * fma_rn(q.w, t.x, tt.x), T(2) * fma_rn(q.w, t.y, tt.y), T(2) * fma_rn(q.w, t.z, tt.z)};
 }
 template <class T>
 DL_HD V3<T> qrot(Q4<T> q, V3<T> v) {
@@ -170,6 +202,48 @@ DL_HD V3<T> qlog(Q4<T> q) {
   T f = (s < tiny_angle<T>()) ? T(2) / q.w : T(2) * dl_atan2(s, q.w) / s;
   return f * u;
 }
+// qlog and qexp of the moderate rotations that an element's two ends or its
+// Gauss points are apart.  log: phi = 2 atan(t)/t u/w with t = |u|/w, by the
+// series of atan(t)/t in t^2 while t^2 is below the limit to which it is exact
+// to rounding (0.03, angles to 0.34, FP32: five terms leave 2e-9; 0.01, angles to
+// 0.2, FP64: eight terms leave 6e-18); no square root, no atan2, one division.
+// exp: the series of cos(t/2) and sin(t/2)/t in t^2 <= 0.04.  Larger angles
+// take the general functions.
+DL_HD float atan_ratio(float t2) {
+  return 1.0f + t2 * (-1.0f / 3 + t2 * (1.0f / 5 + t2 * (-1.0f / 7 + t2 * (1.0f / 9))));
+}
+DL_HD double atan_ratio(double t2) {
+  const double t4 = t2 * t2;
+  const double a = 1.0 + t2 * (-1.0 / 3), b = 1.0 / 5 + t2 * (-1.0 / 7);
+  const double c = 1.0 / 9 + t2 * (-1.0 / 11), d = 1.0 / 13 + t2 * (-1.0 / 15);
+  return (a + t4 * b) + (t4 * t4) * (c + t4 * d);
+}
+DL_HD float atan_ratio_limit(float) { return 0.03f; }
+DL_HD double atan_ratio_limit(double) { return 0.01; }
+template <class T>
+DL_HD V3<T> qlog_near(Q4<T> q) {
+  const V3<T> u{q.x, q.y, q.z};
+  const T s2 = dot(u, u);
+  if (!(q.w > T(0) && s2 < atan_ratio_limit(T(0)) * (q.w * q.w))) return qlog(q);
+  const T iw = T(1) / q.w;
+  return (T(2) * iw * atan_ratio(s2 * iw * iw)) * u;
+}
+DL_HD void exp_ratios(float t2, float *c, float *f) {
+  *c = 1.0f + t2 * (-1.0f / 8 + t2 * (1.0f / 384 - t2 * (1.0f / 46080)));
+  *f = 0.5f + t2 * (-1.0f / 48 + t2 * (1.0f / 3840));
+}
+DL_HD void exp_ratios(double t2, double *c, double *f) {
+  *c = 1.0 + t2 * (-1.0 / 8 + t2 * (1.0 / 384 + t2 * (-1.0 / 46080 + t2 * (1.0 / 10321920))));
+  *f = 0.5 + t2 * (-1.0 / 48 + t2 * (1.0 / 3840 + t2 * (-1.0 / 645120 + t2 * (1.0 / 185794560))));
+}
+template <class T>
+DL_HD Q4<T> qexp_near(V3<T> phi) {
+  const T t2 = dot(phi, phi);
+  if (!(t2 < T(0.04))) return qexp(phi);
+  T c, f;
+  exp_ratios(t2, &c, &f);
+  return Q4<T>{c, f * phi.x, f * phi.y, f * phi.z};
+}
 // square root of a unit quaternion with w >= 0: exp(log(q)/2)
 template <class T>
 DL_HD Q4<T> qhalf(Q4<T> q) {
@@ -180,7 +254,7 @@ DL_HD Q4<T> qhalf(Q4<T> q) {
 }
 template <class T>
 DL_HD Q4<T> qnormalize(Q4<T> q) {
-  T i = dl_rsqrt(q.w * q.w + q.x * q.x + q.y * q.y + q.z * q.z);
+  T i = dl_rsqrt(fma_rn(q.z, q.z, fma_rn(q.y, q.y, fma_rn(q.x, q.x, mul_rn(q.w, q.w)))));
   return Q4<T>{q.w * i, q.x * i, q.y * i, q.z * i};
 }
 
@@ -222,7 +296,7 @@ DL_HD ElemKin<T> elem_kin(V3<double> xi, V3<double> xj, Q4<double> Ri, Q4<double
   Q4<double> LJ = qmul(Rj, qNj);
   Q4<double> qIJ = qmul(qconj(LI), LJ);
   if (qIJ.w < 0.0) qIJ = Q4<double>{-qIJ.w, -qIJ.x, -qIJ.y, -qIJ.z};
-  k.phi = qlog(cvtq<T>(qIJ));
+  k.phi = qlog_near(cvtq<T>(qIJ));
   Q4<double> qh = qhalf(qIJ);
   Q4<double> Lr = qmul(LI, qh);
   V3<double> pp = invL0 * (xj - xi);
