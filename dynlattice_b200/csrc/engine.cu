@@ -344,7 +344,7 @@ struct Engine final : EngineBase {
       m.max_iter = h.max_iter;
       m.prec = T(h.prec);
     }
-    upload_records();
+    pack_records();
     ef.alloc(static_cast<size_t>(E) * 6 * h.nen * sizeof(T));  // one 6-value slot per element node
     DL_CUDA(cudaMemset(ef.p, 0, ef.bytes));
     m.ef = ef.as<T>();
@@ -511,56 +511,18 @@ struct Engine final : EngineBase {
     m.ef = ef.as<T>();
   }
 
-  // The records the step kernels read (ElemRecIx, NodeRecIx), from the host model.
-  void upload_records() {
+  // The records the step kernels read (ElemRecIx, NodeRecIx).
+  void pack_records() {
     const HostLattice &h = *host;
-    const int N = h.N, E = h.E, G = h.G;
-    auto ints = [](T *p, int a, int b, int c, int d) {
-      const int32_t v[4] = {a, b, c, d};
-      std::memcpy(p, v, sizeof v);
-    };
     if (h.nen == 2) {
-      using Ix = ElemRecIx<T>;
-      const int nv = Ix::vecs(G);
-      std::vector<T> r(static_cast<size_t>(tiles32(E)) * nv * Vec16<T>::n, T(0));
-      for (int e = 0; e < E; ++e) {
-        auto at = [&](int s) { return r.data() + rec_ix<T>(nv, e, s); };
-        ints(at(Ix::ints), h.conn[2 * e], h.conn[2 * e + 1], h.eslot[2 * e], h.eslot[2 * e + 1]);
-        for (int a = 0; a < 2; ++a)
-          for (int k = 0; k < 4; ++k) *at(Ix::qN + 4 * a + k) = T(h.qN[(static_cast<size_t>(a) * E + e) * 4 + k]);
-        for (int k = 0; k < 6; ++k) *at(Ix::C + k) = T(h.C[static_cast<size_t>(k) * E + e]);
-        for (int k = 0; k < 2; ++k) *at(Ix::ec + k) = T(h.ec[static_cast<size_t>(k) * E + e]);
-        for (int k = 0; k < 3; ++k) *at(Ix::k0 + k) = T(h.k0[static_cast<size_t>(k) * E + e]);
-        *at(Ix::L0) = T(1.0 / h.invL0[e]);
-        std::memcpy(at(Ix::invL0), &h.invL0[e], sizeof(double));
-        for (int g = 0; g < G; ++g)
-          for (int k = 0; k < 3; ++k) *at(Ix::g0 + 3 * g + k) = T(h.g0[(static_cast<size_t>(g) * 3 + k) * E + e]);
-      }
-      upload(erec, r);
+      erec.alloc(static_cast<size_t>(tiles32(h.E)) * ElemRecIx<T>::vecs(h.G) * 16);
+      DL_CUDA(cudaMemset(erec.p, 0, erec.bytes));
       m.erec = erec.as<typename Vec16<T>::type>();
     }
-    using Nx = NodeRecIx<T>;
-    std::vector<T> r(static_cast<size_t>(tiles32(N)) * Nx::vecs * Vec16<T>::n, T(0));
-    for (int n = 0; n < N; ++n) {
-      auto at = [&](int s) { return r.data() + rec_ix<T>(Nx::vecs, n, s); };
-      int first = h.bc_ptr[n], held = 0;
-      bool zero = true;
-      for (int b = first; b < h.bc_ptr[n + 1]; ++b) {
-        zero = zero && h.bc[b].kind == BCD_DIRICHLET && h.bc[b].scale < 0 && h.bc[b].factor == 0.0;
-        held |= 1 << h.bc[b].dof;
-      }
-      if (zero) first = -1 - held;
-      ints(at(Nx::ints), h.slot_ptr[n], h.slot_ptr[n + 1], first, h.bc_ptr[n + 1]);
-      for (int k = 0; k < 4; ++k) *at(Nx::P + k) = T(h.iframe[static_cast<size_t>(n) * 4 + k]);
-      const double im = 1.0 / h.mass[n];
-      std::memcpy(at(Nx::imass), &im, sizeof im);
-      for (int k = 0; k < 3; ++k) {
-        *at(Nx::D + k) = T(h.idiag[static_cast<size_t>(n) * 4 + k]);
-        *at(Nx::Dinv + k) = T(1.0 / h.idiag[static_cast<size_t>(n) * 4 + k]);
-      }
-    }
-    upload(nrec, r);
+    nrec.alloc(static_cast<size_t>(tiles32(h.N)) * NodeRecIx<T>::vecs * 16);
+    DL_CUDA(cudaMemset(nrec.p, 0, nrec.bytes));
     m.nrec = nrec.as<typename Vec16<T>::type>();
+    DL_CUDA(launch_pack<T>(m, erec.as<T>(), nrec.as<T>(), nullptr));
   }
 
   ~Engine() override {

@@ -94,6 +94,9 @@ cudaError_t launch_milne(const KernelSet &ks, const DevModel<T> &m, const Sample
 // strain; material frame or spatial; out [E][6] internal element order.
 template <class T>
 cudaError_t launch_elem_table(const DevModel<T> &m, int kind, bool spatial, double *out, cudaStream_t s);
+// Packs the step kernels' records (erec null: no two-node elements).
+template <class T>
+cudaError_t launch_pack(const DevModel<T> &m, T *erec, T *nrec, cudaStream_t s);
 // blocks and threads per block of the predictor-corrector launch for a model
 void milne_shape(const KernelSet &ks, int work, int *blocks, int *tpb);
 // Accumulate the per-step external work of a launch into the running total,
