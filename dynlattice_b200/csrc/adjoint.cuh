@@ -544,9 +544,12 @@ DL_HD void elem_vjp_prefix(const ElemIn<T> &in, ElemPrefix<T> &p) {
 // the return-map iterates), then reverses the end-force accumulation, the
 // stress (return map) and the strain into acc.  lh: on entry the adjoint of
 // the point's history after the step, on exit that of the history before it.
-template <class T, class Y, class M>
+// The forward part reads neither lf nor lh: get_adjoints() is called between the
+// two parts and fills them.
+template <class T, class Y, class M, class F>
 DL_HD void elem_vjp_gp(const M &mdl, const PlastLaw<T> &law, const ElemIn<T> &in, const ElemPrefix<T> &p, int g,
-                       const GpIn<T> &gi, const double lf[12], GpHistAdj *lh, double ldiss, ElemGpAdj<T> &acc) {
+                       const GpIn<T> &gi, F &&get_adjoints, const double lf[12], GpHistAdj *lh, double ldiss,
+                       ElemGpAdj<T> &acc) {
   const int G = in.G;
   const ElemKin<T> &k = p.k;
   const T xg = T(adj_gxi(G, g));
@@ -574,6 +577,7 @@ DL_HD void elem_vjp_gp(const M &mdl, const PlastLaw<T> &law, const ElemIn<T> &in
   const T hw = T(0.5) * Wg;
   const T wI = T(wgt) * (T(0.5) * (T(1) - xg));
   const T wJ = T(wgt) * (T(0.5) * (T(1) + xg));
+  get_adjoints();
   // f accumulation reverse
   const V3<T> lfIt{T(lf[0]), T(lf[1]), T(lf[2])}, lfIr{T(lf[3]), T(lf[4]), T(lf[5])};
   const V3<T> lfJt{T(lf[6]), T(lf[7]), T(lf[8])}, lfJr{T(lf[9]), T(lf[10]), T(lf[11])};
@@ -689,7 +693,7 @@ DL_HD void elem_vjp(const M &mdl, const PlastLaw<T> &law, const ElemIn<T> &in, c
       gi.al[a] = in.al[g][a];
       gh.al[a] = lh->al[g][a];
     }
-    elem_vjp_gp<T, Y>(mdl, law, in, p, g, gi, lf, &gh, ldiss[g], acc);
+    elem_vjp_gp<T, Y>(mdl, law, in, p, g, gi, [] {}, lf, &gh, ldiss[g], acc);
     for (int q = 0; q < 6; ++q) {
       lh->ep[g][q] = gh.ep[q];
       lh->epsc[g][q] = gh.epsc[q];

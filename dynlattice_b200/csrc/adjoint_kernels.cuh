@@ -33,23 +33,22 @@ struct AdjElastic {
   __device__ static void vjp(const M &, const T *, T, const T *, T *) {}
 };
 
+// The reverse kernels of consecutive steps wait for one another through the
+// adjoint buffers only; what they read of the tape and recompute from it depends
+// on no earlier one.  So each is launched (programmatic dependent launch) once its
+// predecessor has got through its own wait, does that part meanwhile, and waits
+// here for the predecessor's end: every kernel of the sweep executes this wait, so
+// an end implies the ends of all before it.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Reverse of the node update of one step for node n.
 template <class T>
 __device__ __forceinline__ void adj_node_one(const DevModel<T> &m, const AdjCtx<T> &a, int64_t step, int n) {
   const int N = m.N;
   const size_t s1 = static_cast<size_t>(step - m.tp_step0), s0 = s1 - 1;
-  // complete adjoint of the state after the step
-  double lx1[3] = {a.lx[n], a.lx[N + n], a.lx[2 * N + n]};
-  double lt1[3] = {a.lth[n], a.lth[N + n], a.lth[2 * N + n]};
-  for (int i = m.slot_ptr[n]; i < m.slot_ptr[n + 1]; ++i) {
-    const double *q = a.aslot + static_cast<size_t>(i) * 6;
-    for (int k = 0; k < 3; ++k) {
-      lx1[k] += q[k];
-      lt1[k] += q[3 + k];
-    }
-  }
-  double lv1[6];
-  for (int k = 0; k < 6; ++k) lv1[k] = a.lv[k * N + n];
   NodeIn in;
   const double4 x0 = m.tp_pos[s0 * N + n], r0 = m.tp_rot[s0 * N + n];
   in.x = V3<double>{x0.x, x0.y, x0.z};
@@ -76,6 +75,19 @@ __device__ __forceinline__ void adj_node_one(const DevModel<T> &m, const AdjCtx<
     in.aPre[k] = (v1[k] - in.v[k]) / m.dt;  // the prescribed accelerations of the masked DOFs
     in.fx[k] = 0.0;                           // loads do not enter the adjoint
   }
+  pdl_wait();
+  // complete adjoint of the state after the step
+  double lx1[3] = {a.lx[n], a.lx[N + n], a.lx[2 * N + n]};
+  double lt1[3] = {a.lth[n], a.lth[N + n], a.lth[2 * N + n]};
+  for (int i = m.slot_ptr[n]; i < m.slot_ptr[n + 1]; ++i) {
+    const double *q = a.aslot + static_cast<size_t>(i) * 6;
+    for (int k = 0; k < 3; ++k) {
+      lx1[k] += q[k];
+      lt1[k] += q[3 + k];
+    }
+  }
+  double lv1[6];
+  for (int k = 0; k < 6; ++k) lv1[k] = a.lv[k * N + n];
   double seed[6] = {0, 0, 0, 0, 0, 0};
   if (step == a.peak_step && a.peak_flag && a.peak_flag[n]) seed[a.peak_dof] = a.w_peak;
   V3<double> lx0, lth0;
@@ -101,6 +113,7 @@ __global__ void __launch_bounds__(256) k_adj_node(const __grid_constant__ DevMod
                                                         int64_t step) {
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x)
     adj_node_one(m, a, step, n);
+  pdl_wait();  // also the threads without a node
 }
 
 // sum over the P lanes of an element (lanes aligned to P, P a power of two)
@@ -165,10 +178,6 @@ __global__ void __launch_bounds__(256) k_adj_elem(const __grid_constant__ DevMod
     in.nh = nh;
     in.plastic = m.plastic;
     double lf[12];
-    for (int k = 0; k < 6; ++k) {
-      lf[k] = a.lf[k * N + c.x];
-      lf[6 + k] = a.lf[k * N + c.y];
-    }
     ElemGpAdj<T> acc;
     gp_adj_zero(acc);
     const bool plastic = Y::kPlastic && m.plastic;
@@ -188,16 +197,24 @@ __global__ void __launch_bounds__(256) k_adj_elem(const __grid_constant__ DevMod
         for (int q = 0; q < 6; ++q) {
           gi.ep[q] = th[hist_ix<T>(G, m.hs, e, g, q)];
           gi.epsc[q] = te[epsc_ix(G, e, g, q)];
+        }
+        for (int q = 0; q < nh; ++q) gi.al[q] = th[hist_ix<T>(G, m.hs, e, g, 6 + q)];
+        ldiss = a.w_diss * adj_gw(G, g) * 0.5 * in.L0;
+      }
+      auto adjoints = [&] {
+        pdl_wait();
+        for (int k = 0; k < 6; ++k) {
+          lf[k] = a.lf[k * N + c.x];
+          lf[6 + k] = a.lf[k * N + c.y];
+        }
+        if (!plastic) return;
+        for (int q = 0; q < 6; ++q) {
           lh.ep[q] = a.lep[(g * 6 + q) * E + e];
           lh.epsc[q] = a.lepsc[(g * 6 + q) * E + e];
         }
-        for (int q = 0; q < nh; ++q) {
-          gi.al[q] = th[hist_ix<T>(G, m.hs, e, g, 6 + q)];
-          lh.al[q] = a.lal[(g * nh + q) * E + e];
-        }
-        ldiss = a.w_diss * adj_gw(G, g) * 0.5 * in.L0;
-      }
-      elem_vjp_gp<T, Y>(m, law, in, pre, g, gi, lf, &lh, ldiss, acc);
+        for (int q = 0; q < nh; ++q) lh.al[q] = a.lal[(g * nh + q) * E + e];
+      };
+      elem_vjp_gp<T, Y>(m, law, in, pre, g, gi, adjoints, lf, &lh, ldiss, acc);
       if (plastic) {
         for (int q = 0; q < 6; ++q) {
           a.lep[(g * 6 + q) * E + e] = lh.ep[q];
@@ -237,6 +254,7 @@ __global__ void __launch_bounds__(256) k_adj_elem(const __grid_constant__ DevMod
       a.lec[E + e] += o.lec[1];
     }
   }
+  pdl_wait();  // also the threads without a Gauss point
 }
 
 }  // namespace dl

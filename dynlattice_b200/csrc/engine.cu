@@ -1395,8 +1395,22 @@ struct Engine final : EngineBase {
       for (int64_t k = base + c * K + len; k > base + c * K; --k) {
         int64_t kk = k;
         void *args[] = {&mt, &a, &kk};
-        DL_CUDA(cudaLaunchKernel(ak.node, dim3(nb), dim3(tn), args, 0, rstream));
-        DL_CUDA(cudaLaunchKernel(ak.elem, dim3(eb), dim3(te), args, 0, rstream));
+        // after the segment's first kernel, each may start before the last one ends
+        // (pdl_wait in adjoint_kernels.cuh)
+        cudaLaunchAttribute early{};
+        early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        early.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t lc{};
+        lc.stream = rstream;
+        lc.attrs = &early;
+        lc.numAttrs = k < base + c * K + len ? 1 : 0;
+        lc.gridDim = dim3(nb);
+        lc.blockDim = dim3(tn);
+        DL_CUDA(cudaLaunchKernelExC(&lc, ak.node, args));
+        lc.numAttrs = 1;
+        lc.gridDim = dim3(eb);
+        lc.blockDim = dim3(te);
+        DL_CUDA(cudaLaunchKernelExC(&lc, ak.elem, args));
         adj_launches += 2;
       }
       if (!full) {
