@@ -48,10 +48,11 @@ int threads_for(int work);
 
 // Models of at most this many elements, nodes and pairs run in one block, whose
 // own barrier then replaces the grid's: two grid barriers are 3.5 us of a step.
-// FP64 rods, us per step, several blocks against one: 33 nodes 8.7 / 5.3, 128
-// nodes 10.2 / 5.8, 249 nodes (two items per thread) 9.3 / 8.6; an elastoplastic
+// With the two-barrier kernels, FP64 rods, us per step, several blocks against
+// one: 33 nodes 8.7 / 5.3, 128 nodes 10.2 / 5.8, 249 nodes (two items per thread) 9.3 / 8.6; an elastoplastic
 // 2^3 BCC lattice (163 nodes, 128 elements) 14.0 / 9.6.  Above that the one SM's
-// FP64 units and the items each thread walks cost what the barriers did.
+// FP64 units and the items each thread walks cost what the barriers did.  The
+// one-barrier kernel takes the same line (33 nodes 3.4, 251 nodes 5.7 in one block).
 constexpr int kSoloWork = 256;
 
 // Entry points of the two reverse-step kernels (adjoint_kernels.cuh).

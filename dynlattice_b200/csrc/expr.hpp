@@ -47,7 +47,8 @@ void runProgram(const ExprProgram &p, const double *args, double *out);
 
 // CUDA source of the yield-function policy `YieldJit` for the step kernels:
 // straight-line code (common subexpressions shared) for f(args) and for the
-// gradient list, in float (fp32) or double.
+// gradient list, in float (fp32) or double; what depends on the element's own
+// variables alone comes from prep() and prep_grad(), once per element or flow.
 std::string emitYieldPolicy(const ExprPtr &f, const std::vector<ExprPtr> &grads, bool fp32);
 
 // Source of the policy `YieldAdj` of the adjoint kernels: f and the gradient

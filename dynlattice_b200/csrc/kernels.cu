@@ -129,8 +129,19 @@ void set_persistent_caps(KernelSet &ks) {
 }
 
 int resident_blocks(const void *kernel, int threads, size_t smem) {
-  int occ = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+  // the kernel's limit goes to what a block can have at all, not to this model's
+  // size: it belongs to the kernel, which models of other sizes use too
+  cudaFuncAttributes fa{};
+  int dev = 0, most = 0, occ = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  most -= static_cast<int>(fa.sharedSizeBytes);
+  if (most < 0 || smem > static_cast<size_t>(most)) return 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;

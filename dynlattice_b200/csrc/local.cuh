@@ -17,8 +17,10 @@
 // What bounds the step is latency, not bandwidth: a grid barrier is 1.7 us, a
 // dependent round trip to L2 0.4 us.  Against the two-barrier kernel (step.cuh),
 // which reads every node state from L2 in both phases, this one drops a
-// barrier, the gathers and the state loads of a step for some 10 to 50 % more
-// node updates.
+// barrier, the gathers and the state loads of a step for 10 to 50 % more node
+// updates.  us per step, two barriers against one: 4^3 BCC 9.7 / 6.1, 8^3 10.5 / 6.3
+// (FP64 12.4 / 6.4), 5^3 octet FP64 9.0 / 5.7, 17^3 SC 9.1 / 6.2, 20^3 BCC (two blocks
+// per SM) 22.7 / 19.7 and FP64 37.4 / 33.8.
 #pragma once
 
 #include "step.cuh"

@@ -78,3 +78,20 @@ def test_barrier_failure_is_reported_and_cleared(gpu):
     g.clear_error()
     g.run(4)
     g.synchronize()
+
+
+def test_models_of_different_sizes_side_by_side(gpu):
+    """Each model's launches take their own shared memory, whatever was created
+    after it."""
+    big = Lattice(_spec("bcc", 12, 2, 2, False), DL_MIXED)
+    ref = Lattice(_spec("bcc", 12, 2, 2, False), DL_MIXED)
+    ref.run(10)
+    ref.synchronize()
+    small = Lattice(_spec("bcc", 4, 2, 2, False), DL_MIXED)
+    for _ in range(5):
+        small.run(2)
+        big.run(2)
+    small.synchronize()
+    big.synchronize()
+    for x, y in zip(big.state(), ref.state()):
+        assert np.array_equal(x, y)
