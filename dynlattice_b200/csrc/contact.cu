@@ -75,9 +75,12 @@ __global__ void k_pairs(const double4 *pos, const int2 *conn, const int32_t *rod
                         const unsigned *start, const unsigned *count, const int *items, unsigned mask,
                         const int32_t *nr_ptr, const int32_t *nr, const unsigned long long *bl, int nbl,
                         double reach, int2 *pairs, unsigned cap, unsigned *n_pairs) {
-  // threads walk the elements in bucket order (items), so neighbouring
-  // threads query the same cells
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < E; t += gridDim.x * blockDim.x) {
+  // nine threads per element, one for each row of three cells: a thread's walk is
+  // a chain of dependent loads.  Threads take the elements in bucket order
+  // (items), so neighbouring threads query the same cells.
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 9 * E; i += gridDim.x * blockDim.x) {
+    const int row = i / E, t = i - row * E;
+    const int dz = row / 3 - 1, dy = row % 3 - 1;
     const int e = items[t];
     const int4 ce = cell[e];
     const int2 ce2 = conn[e];
@@ -88,38 +91,36 @@ __global__ void k_pairs(const double4 *pos, const int2 *conn, const int32_t *rod
     g.A[1][0] = a1.x; g.A[1][1] = a1.y; g.A[1][2] = a1.z;
     const double alo[3] = {fmin(a0.x, a1.x) - reach, fmin(a0.y, a1.y) - reach, fmin(a0.z, a1.z) - reach};
     const double ahi[3] = {fmax(a0.x, a1.x) + reach, fmax(a0.y, a1.y) + reach, fmax(a0.z, a1.z) + reach};
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int ix = ce.x + dx, iy = ce.y + dy, iz = ce.z + dz;
-          const unsigned key = cell_hash(ix, iy, iz, mask);
-          const unsigned s0 = start[key], n = count[key];
-          for (unsigned q = 0; q < n; ++q) {
-            const int f = items[s0 + q];
-            if (f <= e) continue;
-            const int4 cf = cell[f];
-            if (cf.x != ix || cf.y != iy || cf.z != iz) continue;  // other cell in the same bucket
-            const int rf = rod[f];
-            if (rf == re) continue;
-            const int2 cf2 = conn[f];
-            const double4 b0 = pos[cf2.x], b1 = pos[cf2.y];
-            // bounding boxes (inflated by the reach) must overlap
-            if (fmax(b0.x, b1.x) < alo[0] || fmin(b0.x, b1.x) > ahi[0] || fmax(b0.y, b1.y) < alo[1] ||
-                fmin(b0.y, b1.y) > ahi[1] || fmax(b0.z, b1.z) < alo[2] || fmin(b0.z, b1.z) > ahi[2])
-              continue;
-            g.B[0][0] = b0.x; g.B[0][1] = b0.y; g.B[0][2] = b0.z;
-            g.B[1][0] = b1.x; g.B[1][1] = b1.y; g.B[1][2] = b1.z;
-            if (segment_distance(g) > reach) continue;
-            if (node_in_rod(nr_ptr, nr, ce2.x, rf) || node_in_rod(nr_ptr, nr, ce2.y, rf) ||
-                node_in_rod(nr_ptr, nr, cf2.x, re) || node_in_rod(nr_ptr, nr, cf2.y, re))
-              continue;
-            // orientation of the reference: A belongs to the rod with the smaller index
-            const int pa = (re < rf) ? e : f, pb = (re < rf) ? f : e;
-            if (nbl > 0 && blacklisted(bl, nbl, pa, pb)) continue;
-            const unsigned slot = atomicAdd(n_pairs, 1u);
-            if (slot < cap) pairs[slot] = make_int2(pa, pb);
-          }
-        }
+    for (int dx = -1; dx <= 1; ++dx) {
+      const int ix = ce.x + dx, iy = ce.y + dy, iz = ce.z + dz;
+      const unsigned key = cell_hash(ix, iy, iz, mask);
+      const unsigned s0 = start[key], n = count[key];
+      for (unsigned q = 0; q < n; ++q) {
+        const int f = items[s0 + q];
+        if (f <= e) continue;
+        const int4 cf = cell[f];
+        if (cf.x != ix || cf.y != iy || cf.z != iz) continue;  // other cell in the same bucket
+        const int rf = rod[f];
+        if (rf == re) continue;
+        const int2 cf2 = conn[f];
+        const double4 b0 = pos[cf2.x], b1 = pos[cf2.y];
+        // bounding boxes (inflated by the reach) must overlap
+        if (fmax(b0.x, b1.x) < alo[0] || fmin(b0.x, b1.x) > ahi[0] || fmax(b0.y, b1.y) < alo[1] ||
+            fmin(b0.y, b1.y) > ahi[1] || fmax(b0.z, b1.z) < alo[2] || fmin(b0.z, b1.z) > ahi[2])
+          continue;
+        g.B[0][0] = b0.x; g.B[0][1] = b0.y; g.B[0][2] = b0.z;
+        g.B[1][0] = b1.x; g.B[1][1] = b1.y; g.B[1][2] = b1.z;
+        if (segment_distance(g) > reach) continue;
+        if (node_in_rod(nr_ptr, nr, ce2.x, rf) || node_in_rod(nr_ptr, nr, ce2.y, rf) ||
+            node_in_rod(nr_ptr, nr, cf2.x, re) || node_in_rod(nr_ptr, nr, cf2.y, re))
+          continue;
+        // orientation of the reference: A belongs to the rod with the smaller index
+        const int pa = (re < rf) ? e : f, pb = (re < rf) ? f : e;
+        if (nbl > 0 && blacklisted(bl, nbl, pa, pb)) continue;
+        const unsigned slot = atomicAdd(n_pairs, 1u);
+        if (slot < cap) pairs[slot] = make_int2(pa, pb);
+      }
+    }
   }
 }
 
@@ -138,14 +139,27 @@ __global__ void k_closed(const double4 *pos, const int2 *conn, const int2 *pairs
   }
 }
 
-__global__ void k_max_speed(const double *vel, int N, unsigned long long *out) {
-  double m = 0.0;
+// largest node speed, and largest distance of a node from x (null: 0), as the
+// bits of out[0] and out[1]
+__global__ void k_motion(const double *vel, const double4 *pos, const double *x, int N, unsigned long long *out) {
+  double m = 0.0, d2 = 0.0;
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
     const double a = vel[vel_ix(n, 0)], b = vel[vel_ix(n, 1)], c = vel[vel_ix(n, 2)];
     m = fmax(m, sqrt(a * a + b * b + c * c));
+    if (x) {
+      const double4 p = pos[n];
+      const double dx = p.x - x[3 * n], dy = p.y - x[3 * n + 1], dz = p.z - x[3 * n + 2];
+      d2 = fmax(d2, dx * dx + dy * dy + dz * dz);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __double_as_longlong(m));
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+    d2 = fmax(d2, __shfl_down_sync(0xffffffffu, d2, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(out, __double_as_longlong(m));
+    if (x) atomicMax(out + 1, __double_as_longlong(sqrt(d2)));
+  }
 }
 
 __global__ void k_copy_xyz(const double4 *pos, int N, double *x) {
@@ -354,7 +368,7 @@ void ContactList::init(const HostLattice &h, cudaStream_t s) {
   start.alloc(static_cast<size_t>(T) * sizeof(unsigned));
   cursor.alloc(static_cast<size_t>(T) * sizeof(unsigned));
   items.alloc(static_cast<size_t>(E) * sizeof(int));
-  scalars.alloc(4 * sizeof(unsigned long long));
+  scalars.alloc(5 * sizeof(unsigned long long));
   xbuild.alloc(static_cast<size_t>(N) * 3 * sizeof(double));
   size_t tmp = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, tmp, static_cast<unsigned *>(nullptr), static_cast<unsigned *>(nullptr),
@@ -381,7 +395,7 @@ void ContactList::build(const double4 *pos, const int2 *conn, double reach) {
     k_fill<<<blocks_for(E), 256, 0, stream>>>(cell.as<int4>(), E, start.as<unsigned>(), cursor.as<unsigned>(),
                                               items.as<int>());
     unsigned *npair = reinterpret_cast<unsigned *>(sc + 1);
-    k_pairs<<<blocks_for(E), 256, 0, stream>>>(pos, conn, rod.as<int32_t>(), E, cell.as<int4>(),
+    k_pairs<<<blocks_for(9 * E), 256, 0, stream>>>(pos, conn, rod.as<int32_t>(), E, cell.as<int4>(),
                                                start.as<unsigned>(), count.as<unsigned>(), items.as<int>(), mask,
                                                nr_ptr.as<int32_t>(), nr.as<int32_t>(),
                                                blacklist.as<unsigned long long>(), n_blacklist, reach,
@@ -449,19 +463,6 @@ void ContactList::init_blacklist(const double4 *pos, const int2 *conn) {
   }
 }
 
-double ContactList::max_speed(const double *vel) {
-  unsigned long long *sc = scalars.as<unsigned long long>();
-  check(cudaMemsetAsync(sc + 3, 0, sizeof(unsigned long long), stream), "memset");
-  k_max_speed<<<blocks_for(N), 256, 0, stream>>>(vel, N, sc + 3);
-  ++launches;
-  unsigned long long bits = 0;
-  check(cudaMemcpyAsync(&bits, sc + 3, sizeof bits, cudaMemcpyDeviceToHost, stream), "readback");
-  check(cudaStreamSynchronize(stream), "sync");
-  double v;
-  std::memcpy(&v, &bits, sizeof v);
-  return v;
-}
-
 void JointList::init(const HostLattice &h, cudaStream_t s) {
   stream = s;
   N = h.N;
@@ -488,7 +489,7 @@ void JointList::init(const HostLattice &h, cudaStream_t s) {
   start.alloc(static_cast<size_t>(T) * sizeof(unsigned));
   cursor.alloc(static_cast<size_t>(T) * sizeof(unsigned));
   items.alloc(Jn * sizeof(int));
-  scalars.alloc(4 * sizeof(unsigned long long));
+  scalars.alloc(5 * sizeof(unsigned long long));
   xbuild.alloc(static_cast<size_t>(N) * 3 * sizeof(double));
   size_t tmp = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, tmp, static_cast<unsigned *>(nullptr), static_cast<unsigned *>(nullptr),
@@ -552,15 +553,17 @@ void JointList::build(const double4 *pos) {
   throw std::runtime_error("joint contact candidate list could not be built");
 }
 
-double node_max_speed(const double *vel, int N, unsigned long long *scratch, cudaStream_t stream) {
-  check(cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), stream), "memset");
-  k_max_speed<<<blocks_for(N), 256, 0, stream>>>(vel, N, scratch);
-  unsigned long long bits = 0;
-  check(cudaMemcpyAsync(&bits, scratch, sizeof bits, cudaMemcpyDeviceToHost, stream), "readback");
+NodeMotion node_motion(const double *vel, const double4 *pos, const double *x, int N, unsigned long long *scratch,
+                       cudaStream_t stream) {
+  check(cudaMemsetAsync(scratch, 0, 2 * sizeof(unsigned long long), stream), "memset");
+  k_motion<<<blocks_for(N), 256, 0, stream>>>(vel, pos, x, N, scratch);
+  unsigned long long bits[2] = {0, 0};
+  check(cudaMemcpyAsync(bits, scratch, sizeof bits, cudaMemcpyDeviceToHost, stream), "readback");
   check(cudaStreamSynchronize(stream), "sync");
-  double v;
-  std::memcpy(&v, &bits, sizeof v);
-  return v;
+  NodeMotion r;
+  std::memcpy(&r.speed, &bits[0], sizeof r.speed);
+  std::memcpy(&r.moved, &bits[1], sizeof r.moved);
+  return r;
 }
 
 }  // namespace dl

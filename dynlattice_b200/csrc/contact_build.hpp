@@ -130,7 +130,6 @@ struct ContactList {
   void build(const double4 *pos, const int2 *conn, double reach);
   // pairs already in contact in the initial configuration (computeBlacklist_)
   void init_blacklist(const double4 *pos, const int2 *conn);
-  double max_speed(const double *vel);
 };
 
 // Candidate list of the joint contact (JointContactModel): joint pairs within
@@ -156,6 +155,11 @@ struct JointList {
 };
 
 // max_n |v_n| (translations, [6][N] layout) through `scratch` (one word); synchronises `stream`
-double node_max_speed(const double *vel, int N, unsigned long long *scratch, cudaStream_t stream);
+// Largest speed of a node, and how far one is from the positions x (null: 0).
+struct NodeMotion {
+  double speed = 0.0, moved = 0.0;
+};
+NodeMotion node_motion(const double *vel, const double4 *pos, const double *x, int N, unsigned long long *scratch,
+                       cudaStream_t stream);
 
 }  // namespace dl

@@ -1808,7 +1808,9 @@ __device__ __forceinline__ void element_phase(const DevModel<T> &m, const Sample
   }
   double econ = 0.0;
   if (X) {
-    for (int p = gtid; p < m.n_pairs; p += gstride) contact_pair(m, p, step, energy, econ);
+    // on from the threads that have an element less
+    for (int p = (gtid + gstride - m.E % gstride) % gstride; p < m.n_pairs; p += gstride)
+      contact_pair(m, p, step, energy, econ);
     for (int p = gtid; p < m.n_jpairs; p += gstride) joint_pair(m, p, step, energy, econ);
   }
   if (energy) {
