@@ -122,6 +122,7 @@ struct EngineBase {
   virtual void set_tape_budget(int64_t bytes) = 0;
   virtual void autotune(int64_t steps, int32_t *best_mode, int32_t *best_tpb, double *best_ms) = 0;
   virtual void set_threads(int tpb) = 0;
+  virtual StepLaunch launch_shape(int64_t nsteps) = 0;
   virtual void set_group_output(bool on) = 0;
   virtual void set_integrator(const dl_integrator_desc &d) = 0;
   virtual bool adaptive() const = 0;
@@ -662,6 +663,9 @@ struct Engine final : EngineBase {
   }
 
   void set_threads(int tpb) override { kernels.tpb_override = tpb; }
+  StepLaunch launch_shape(int64_t nsteps) override {
+    return step_launch<T>(kernels, m, nsteps, exec_mode, local);
+  }
   // Recording the internal force of each launch's last step costs a
   // store per node and selects the extended kernel variant, so it is off
   // until a caller asks for group sums.
@@ -675,11 +679,11 @@ struct Engine final : EngineBase {
 
   // ---- autotuner -------------------------------------------------------------
   // Times `steps` steps of a fresh copy of this lattice for each launch shape
-  // (persistent launch with 32..256 threads per block, two launches per step)
-  // and keeps the fastest for this handle.
+  // (the automatic one, the persistent launch with 32..256 threads per block, two
+  // launches per step) and keeps the fastest for this handle.
   void autotune(int64_t steps, int32_t *best_mode, int32_t *best_tpb, double *best_ms) {
-    const int cand[5][2] = {{EXEC_PERSISTENT, 256}, {EXEC_PERSISTENT, 128}, {EXEC_PERSISTENT, 64},
-                            {EXEC_PERSISTENT, 32}, {EXEC_STREAM, 0}};
+    const int cand[6][2] = {{EXEC_PERSISTENT, 0}, {EXEC_PERSISTENT, 256}, {EXEC_PERSISTENT, 128},
+                            {EXEC_PERSISTENT, 64}, {EXEC_PERSISTENT, 32}, {EXEC_STREAM, 0}};
     cudaEvent_t a, b;
     DL_CUDA(cudaEventCreate(&a));
     DL_CUDA(cudaEventCreate(&b));
@@ -1946,6 +1950,18 @@ DL_API int dl_set_threads(dl_handle *h, int32_t threads) {
   if (!h || !(threads == 0 || threads == 32 || threads == 64 || threads == 128 || threads == 256))
     return set_err(DL_ERR_INVALID, "threads per block must be 0 (automatic), 32, 64, 128 or 256");
   return guard([&] { h->eng->set_threads(threads); });
+}
+
+DL_API int dl_get_launch_shape(dl_handle *h, int64_t nsteps, int32_t *kernel, int32_t *blocks, int32_t *threads,
+                               int64_t *shared_bytes) {
+  if (!h || nsteps <= 0) return set_err(DL_ERR_INVALID, "bad argument");
+  return guard([&] {
+    const dl::StepLaunch l = h->eng->launch_shape(nsteps);
+    if (kernel) *kernel = l.kind;
+    if (blocks) *blocks = l.blocks;
+    if (threads) *threads = l.threads;
+    if (shared_bytes) *shared_bytes = static_cast<int64_t>(l.smem);
+  });
 }
 
 DL_API int dl_autotune(dl_handle *h, int64_t steps, int32_t *best_mode, int32_t *best_threads, double *best_ms) {

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "../../include/dynlattice.h"
 #include "devtypes.cuh"
 
 namespace dl {
@@ -81,6 +82,23 @@ struct LocalLaunch {
 };
 // Blocks of `threads` threads and `smem` bytes that are resident on an SM (0 if none).
 int resident_blocks(const void *kernel, int threads, size_t smem);
+// Whether a launch takes the extended kernels: only when the model or the run
+// uses their features.
+template <class T>
+bool extended_run(const DevModel<T> &m) {
+  return m.c_ptr || m.j_ptr || m.n_plates > 0 || m.tp_pos || m.tp_hist || m.grp_hist || m.fint_last || m.br ||
+         m.lumped || m.tie_ptr || m.nen > 2;
+}
+// The kernel and launch shape of a block of nsteps steps (EXEC_STREAM: of the
+// element launches).
+struct StepLaunch {
+  dl_step_kernel kind = DL_STEP_TWO_BARRIERS;
+  const void *kernel = nullptr;
+  int blocks = 0, threads = 0;
+  size_t smem = 0;
+};
+template <class T>
+StepLaunch step_launch(const KernelSet &ks, const DevModel<T> &m, int64_t nsteps, int mode, const LocalLaunch &local);
 template <class T>
 cudaError_t launch_steps(const KernelSet &ks, const DevModel<T> &m, const SampleSpec &smp, const StepCtx &c,
                          int mode, GridBarrier *bar, const LocalLaunch &local, cudaStream_t s);

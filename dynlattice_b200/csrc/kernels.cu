@@ -190,41 +190,61 @@ KernelSet aot_kernels(bool plastic) {
 }
 
 template <class T>
+StepLaunch step_launch(const KernelSet &ks, const DevModel<T> &m, int64_t nsteps, int mode, const LocalLaunch &local) {
+  StepLaunch l;
+  const bool ext = extended_run(m);
+  if (mode == EXEC_STREAM) {
+    l.kind = DL_STEP_TWO_LAUNCHES;
+    l.kernel = ext ? ks.element_x : ks.element;
+    l.blocks = grid_for(m.E, 256);
+    l.threads = 256;
+    return l;
+  }
+  if (local.blocks > 0 && !ext && nsteps > 1 && ks.tpb_override <= 0) {
+    l.kind = DL_STEP_ONE_BARRIER;
+    l.kernel = local.kernel;
+    l.blocks = local.blocks;
+    l.threads = local.threads;
+    l.smem = local.smem;
+    return l;
+  }
+  // one element or node per thread at most: small models take few blocks,
+  // which keeps the grid barriers short
+  const int work = std::max(std::max(m.E, m.N), m.n_pairs);
+  const bool solo = ks.tpb_override <= 0 && work <= kSoloWork;
+  int tpb = ks.tpb_override > 0 ? ks.tpb_override : threads_for(work);
+  if (solo) {
+    tpb = 32;
+    while (tpb < work && tpb < 128) tpb *= 2;
+  } else if (tpb == 256) {
+    tpb = ext ? ks.full_threads_x : ks.full_threads;
+  }
+  const int ci = tpb == 32 ? 0 : (tpb == 64 ? 1 : (tpb == 128 ? 2 : 3));
+  const int want = solo ? 1 : std::max(1, (work + tpb - 1) / tpb);
+  // a launch of one step reports its energies: the kernel with that known
+  const bool one = !ext && nsteps == 1 && ks.persistent1 && ks.persist_cap1[ci] > 0;
+  const int cap = ext ? ks.persist_cap_x[ci] : (one ? ks.persist_cap1[ci] : ks.persist_cap[ci]);
+  l.kind = ext ? DL_STEP_TWO_BARRIERS_X : (one ? DL_STEP_ONE_STEP : DL_STEP_TWO_BARRIERS);
+  l.kernel = ext ? ks.persistent_x : (one ? ks.persistent1 : ks.persistent);
+  l.blocks = std::min(cap > 0 ? cap : ks.persist_blocks, want);
+  l.threads = tpb;
+  return l;
+}
+
+template <class T>
 cudaError_t launch_steps(const KernelSet &ks, const DevModel<T> &m, const SampleSpec &smp, const StepCtx &c,
                          int mode, GridBarrier *bar, const LocalLaunch &local, cudaStream_t s) {
   if (c.nsteps <= 0) return cudaSuccess;
-  // the extended kernels only when the model or the run uses their features
-  const bool ext = m.c_ptr || m.j_ptr || m.n_plates > 0 || m.tp_pos || m.tp_hist || m.grp_hist || m.fint_last ||
-                   m.br || m.lumped || m.tie_ptr || m.nen > 2;
+  const bool ext = extended_run(m);
   DevModel<T> mm = m;
   SampleSpec ss = smp;
   StepCtx cc = c;
   if (mode == EXEC_PERSISTENT || mode == EXEC_GRAPH) {
+    const StepLaunch l = step_launch(ks, m, c.nsteps, mode, local);
     GridBarrier *bb = bar;
-    if (local.blocks > 0 && !ext && c.nsteps > 1 && ks.tpb_override <= 0) {
-      LocalPlan pl = local.plan;
-      void *la[] = {&mm, &ss, &cc, &bb, &pl};
-      return cudaLaunchCooperativeKernel(local.kernel, dim3(local.blocks), dim3(local.threads), la, local.smem, s);
-    }
-    void *args[] = {&mm, &ss, &cc, &bb};
-    // one element or node per thread at most: small models take few blocks,
-    // which keeps the grid barriers short
-    const int work = std::max(std::max(m.E, m.N), m.n_pairs);
-    int tpb = ks.tpb_override > 0 ? ks.tpb_override : threads_for(work);
-    if (ks.tpb_override <= 0 && work <= kSoloWork) {
-      tpb = 32;
-      while (tpb < work && tpb < 128) tpb *= 2;
-    } else if (tpb == 256) {
-      tpb = ext ? ks.full_threads_x : ks.full_threads;
-    }
-    const int ci = tpb == 32 ? 0 : (tpb == 64 ? 1 : (tpb == 128 ? 2 : 3));
-    const int want = ks.tpb_override <= 0 && work <= kSoloWork ? 1 : std::max(1, (work + tpb - 1) / tpb);
-    // a launch of one step reports its energies: the kernel with that known
-    const bool one = !ext && c.nsteps == 1 && ks.persistent1 && ks.persist_cap1[ci] > 0;
-    const int cap = ext ? ks.persist_cap_x[ci] : (one ? ks.persist_cap1[ci] : ks.persist_cap[ci]);
-    const int blocks = std::min(cap > 0 ? cap : ks.persist_blocks, want);
-    const void *kern = ext ? ks.persistent_x : (one ? ks.persistent1 : ks.persistent);
-    return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(tpb), args, 0, s);
+    LocalPlan pl = local.plan;
+    void *args[] = {&mm, &ss, &cc, &bb, &pl};  // the plan: read by the one-barrier kernel only
+    return cudaLaunchCooperativeKernel(l.kernel, dim3(l.blocks), dim3(l.threads), args, l.smem, s);
   }
   const int eb = grid_for(m.E, 256), nb = grid_for(m.N, 256);
   k_clear5<<<1, 32, 0, s>>>(c.last_energy);
@@ -432,6 +452,7 @@ cudaError_t launch_state_in(double4 *pos, double4 *rot, double *vel, const doubl
 
 #define DL_INSTANTIATE(T)                                                                              \
   template KernelSet aot_kernels<T>(bool);                                                                 \
+  template StepLaunch step_launch<T>(const KernelSet &, const DevModel<T> &, int64_t, int, const LocalLaunch &); \
   template cudaError_t launch_steps<T>(const KernelSet &, const DevModel<T> &, const SampleSpec &,     \
                                        const StepCtx &, int, GridBarrier *, const LocalLaunch &,           \
                                        cudaStream_t);                                                 \

@@ -78,6 +78,7 @@ def load_library():
     lib.dl_set_tape_budget.argtypes = [P, C.c_int64]
     lib.dl_autotune.argtypes = [P, C.c_int64, i32p, i32p, dp]
     lib.dl_set_threads.argtypes = [P, C.c_int32]
+    lib.dl_get_launch_shape.argtypes = [P, C.c_int64, i32p, i32p, i32p, C.POINTER(C.c_int64)]
     lib.dl_set_group_output.argtypes = [P, C.c_int32]
     lib.dl_set_integrator.argtypes = [P, C.POINTER(dl_integrator_desc)]
     lib.dl_get_time.argtypes = [P, dp, dp, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
@@ -116,6 +117,7 @@ def trim_retained_memory():
     _check(lib, lib.dl_trim_retained_memory())
 
 
+STEP_KERNELS = ("two_barriers", "one_step", "one_barrier", "two_barriers_x", "two_launches")
 VTU_FINT, VTU_FEXT, VTU_FRES = 1, 2, 4
 
 
@@ -387,10 +389,18 @@ class Lattice:
 
     def autotune(self, steps: int = 200):
         """Pick the fastest launch shape for this lattice (dl_autotune):
-        returns (exec mode, threads per block, ms for `steps` steps)."""
+        returns (exec mode, threads per block, 0 in mode 0 being the automatic shape,
+        ms for `steps` steps)."""
         mode, tpb, ms = C.c_int32(), C.c_int32(), C.c_double()
         self._c(self.lib.dl_autotune(self.h, int(steps), C.byref(mode), C.byref(tpb), C.byref(ms)))
         return mode.value, tpb.value, ms.value
+
+    def launch_shape(self, nsteps: int = 2) -> dict:
+        """The launch that run(nsteps) makes (dl_get_launch_shape): kernel (one of
+        STEP_KERNELS), blocks, threads per block, bytes of dynamic shared memory."""
+        k, b, t, s = C.c_int32(), C.c_int32(), C.c_int32(), C.c_int64()
+        self._c(self.lib.dl_get_launch_shape(self.h, int(nsteps), C.byref(k), C.byref(b), C.byref(t), C.byref(s)))
+        return {"kernel": STEP_KERNELS[k.value], "blocks": b.value, "threads": t.value, "shared_bytes": s.value}
 
     def set_launch_shape(self, mode: int, threads: int):
         """Exec mode and threads per block (e.g. an autotune result)."""

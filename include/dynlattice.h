@@ -378,16 +378,35 @@ DL_API int dl_set_exec_mode(dl_handle *h, int mode);
 
 /* Autotuner (engine extension): times dl_run calls of `steps` steps (at
  * least 50 steps in all) on a fresh copy of the lattice for each launch shape
- * (persistent launch with 256/128/64/32 threads per block, two launches per
- * step) and keeps the fastest for this handle.  Outputs (optional): the
- * chosen mode, threads per block (0 = per-step kernels) and its time per call
- * in ms. */
+ * (the automatic shape, the persistent launch with 256/128/64/32 threads per
+ * block, two launches per step) and keeps the fastest for this handle.  Outputs
+ * (optional): the chosen mode, threads per block (0 in mode 0: the automatic
+ * shape; 0 in mode 1: per-step kernels) and its time per call in ms. */
 DL_API int dl_autotune(dl_handle *h, int64_t steps, int32_t *best_mode,
                        int32_t *best_threads, double *best_ms);
 
-/* Threads per block of the persistent launch: 0 = automatic (256, halved
- * while the grid would not cover every SM), or 32/64/128/256. */
+/* Threads per block of the persistent launch: 0 = automatic, or
+ * 32/64/128/256.  Automatic: the one-barrier kernel where the model fits it,
+ * else one block for small models, else full blocks, halved while the grid
+ * would not cover every SM.  A number set here is that of the two-barrier
+ * kernels, which then run. */
 DL_API int dl_set_threads(dl_handle *h, int32_t threads);
+
+/* Kernels of the explicit step. */
+typedef enum dl_step_kernel {
+  DL_STEP_TWO_BARRIERS = 0,   /* persistent launch, two grid barriers per step      */
+  DL_STEP_ONE_STEP = 1,       /* the same for a launch of one step                  */
+  DL_STEP_ONE_BARRIER = 2,    /* node copies in shared memory, one grid barrier     */
+  DL_STEP_TWO_BARRIERS_X = 3, /* as 0, with contact, adjoint tape, group output ... */
+  DL_STEP_TWO_LAUNCHES = 4    /* exec mode 1: two launches per step                 */
+} dl_step_kernel;
+
+/* The launch that dl_run of nsteps steps (explicit integrator) makes of this
+ * handle as it stands: kernel (dl_step_kernel), blocks, threads per block,
+ * bytes of dynamic shared memory per block.  Any output may be NULL.  Engine
+ * feature; no counterpart in the reference. */
+DL_API int dl_get_launch_shape(dl_handle *h, int64_t nsteps, int32_t *kernel,
+                               int32_t *blocks, int32_t *threads, int64_t *shared_bytes);
 
 /* Advance nsteps explicit steps (LeapFrogModule::solve, LeapFrogModule.cpp:44-84,
  * with ExplicitModule::getForce/getAcce/updateVec, ExplicitModule.cpp:339-419).
