@@ -22,6 +22,7 @@
 #include "../../include/dynlattice.h"
 #include "engine.hpp"
 #include "local.cuh"
+#include "local_plan.hpp"
 #include "jit.hpp"
 #include "noalloc.hpp"
 #include "output.hpp"
@@ -434,20 +435,37 @@ struct Engine final : EngineBase {
       const KernelSet *ks = jit_kernels(code, sizeof(T) == 4, &jit_log);
       if (ks) kernels = *ks;
     }
-    plan_local();
     set_sampling(0, {}, 0);
   }
 
   // The one-barrier kernel's share-out of elements and node copies over the
   // blocks.  One block per SM while the elements of a block stay below its
-  // threads, two above that; a model whose copies do not fit, or that uses what
-  // the kernel does not cover, keeps the two-barrier kernels (blocks = 0).
+  // threads, two above that; a model whose copies do not fit keeps the two-barrier
+  // kernels (blocks = 0).  Made by the first run that can use it: a handle that
+  // differentiates, records group output or steps one by one never does, and the
+  // share-out and its slots cost 0.2 ms at 9,900 elements and 2.3 ms at 128,000.
   LocalLaunch local;
-  DevBuf local_ptr, local_nodes, local_ends;
+  DevBuf local_lists, local_ef;
+  bool local_planned = false;
+  void ensure_plan(int64_t nsteps) {
+    if (local_planned || nsteps < 2 || exec_mode == EXEC_STREAM || kernels.tpb_override > 0 || !kernels.local[0]) return;
+    if (contact_on || joint_on || extended_run(m)) return;
+    // nothing can be allocated while the caller records a graph: this run takes
+    // the two-barrier kernels
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (stream && (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
+      cudaGetLastError();
+      return;
+    }
+    local_planned = true;
+    try {
+      plan_local();
+    } catch (const CudaError &) {  // no memory for it
+      local = LocalLaunch{};
+    }
+  }
   void plan_local() {
     const HostLattice &h = *host;
-    const bool ext = contact_on || joint_on || m.n_plates > 0 || h.lumped || h.ties || h.nen != 2;
-    if (ext || !kernels.local[0]) return;
     const int E = h.E;
     int sms = 0;
     DL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -459,58 +477,36 @@ struct Engine final : EngineBase {
       chunk = std::max(32, (chunk + 7) / 8 * 8);
     }
     const int blocks = (E + chunk - 1) / chunk;
-    // a block of so many elements has too many nodes: spare the set-up the attempt
-    if (static_cast<size_t>(chunk) * sizeof(double) * LocalShape<T>::row / 2 > 232448) return;
-    std::vector<int32_t> ptr(blocks + 1, 0), nodes;
-    std::vector<uint32_t> ends(E);
-    std::vector<int32_t> at(h.N, -1), seen(h.N, -1);
-    int cap = 0;
-    for (int b = 0; b < blocks; ++b) {
-      const int first = static_cast<int>(nodes.size());
-      const int e1 = std::min(E, (b + 1) * chunk);
-      for (int e = b * chunk; e < e1; ++e)
-        for (int a = 0; a < 2; ++a) {
-          const int n = h.conn[2 * e + a];
-          if (seen[n] == b) continue;
-          nodes.push_back(seen[n] < 0 ? static_cast<int32_t>(static_cast<uint32_t>(n) | 0x80000000u) : n);
-          seen[n] = b;
-        }
-      // nodes with equally many slots side by side
-      std::stable_sort(nodes.begin() + first, nodes.end(), [&](int32_t x, int32_t y) {
-        x &= 0x7fffffff;
-        y &= 0x7fffffff;
-        return h.slot_ptr[x + 1] - h.slot_ptr[x] > h.slot_ptr[y + 1] - h.slot_ptr[y];
-      });
-      if (nodes.size() - first > 0xffffu) return;
-      for (size_t i = first; i < nodes.size(); ++i) at[nodes[i] & 0x7fffffff] = static_cast<int32_t>(i) - first;
-      for (int e = b * chunk; e < e1; ++e)
-        ends[e] = static_cast<uint32_t>(at[h.conn[2 * e]]) | (static_cast<uint32_t>(at[h.conn[2 * e + 1]]) << 16);
-      ptr[b + 1] = static_cast<int32_t>(nodes.size());
-      cap = std::max(cap, ptr[b + 1] - ptr[b]);
-    }
-    const int threads = std::min(most, (std::max(std::min(chunk, most), cap) + 31) / 32 * 32);
-    size_t smem = 0;
-    local.kernel = kernels.local[per_sm - 1];
-    for (int recs = 1; recs >= -1; --recs) {
-      if (recs < 0) return;
-      smem = LocalShape<T>::bytes(cap, recs ? chunk : 0, h.G);
-      local.plan.recs = recs;
-      if (resident_blocks(local.kernel, threads, smem) * sms >= blocks) break;
-    }
-    upload(local_ptr, ptr);
-    upload(local_nodes, nodes);
-    upload(local_ends, ends);
-    local.plan.chunk = chunk;
-    local.plan.cap = cap;
-    local.plan.node_ptr = local_ptr.as<int32_t>();
-    local.plan.nodes = local_nodes.as<int32_t>();
-    local.plan.ends = local_ends.as<uint32_t>();
-    local.blocks = blocks;
-    local.threads = threads;
-    local.smem = smem;
-    ef.alloc(static_cast<size_t>(E) * 24 * sizeof(T));  // two sets of end-force slots
-    DL_CUDA(cudaMemset(ef.p, 0, ef.bytes));
-    m.ef = ef.as<T>();
+    LocalLaunch l;
+    l.kernel = kernels.local[per_sm - 1];
+    l.blocks = blocks;
+    // whether blocks of `cap` copies are resident all at once
+    auto fits = [&](int cap, int recs) {
+      l.threads = std::min(most, (std::max(std::min(chunk, most), cap) + 31) / 32 * 32);
+      l.smem = LocalShape<T>::bytes(cap, recs ? chunk : 0, h.G);
+      l.plan.recs = recs;
+      return static_cast<int64_t>(resident_blocks(l.kernel, l.threads, l.smem)) * sms >= blocks;
+    };
+    // every node has a copy in some block: spare larger models the share-out
+    if (!fits((h.N + blocks - 1) / blocks, 0)) return;
+    LocalShare s;
+    share_nodes(h, chunk, blocks, s);
+    if (s.cap > 0xffff || (!fits(s.cap, 1) && !fits(s.cap, 0))) return;
+    share_ends(h, s);
+    // the lists in one array, the second set of end-force slots; on the run's stream
+    std::vector<int32_t> lists(s.ptr);
+    lists.insert(lists.end(), s.nodes.begin(), s.nodes.end());
+    lists.insert(lists.end(), s.ends.begin(), s.ends.end());
+    local_lists.alloc(lists.size() * sizeof(int32_t));
+    local_ef.alloc(static_cast<size_t>(E) * 12 * sizeof(T));
+    DL_CUDA(cudaMemcpyAsync(local_lists.p, lists.data(), local_lists.bytes, cudaMemcpyHostToDevice, stream));
+    l.plan.chunk = chunk;
+    l.plan.cap = s.cap;
+    l.plan.node_ptr = local_lists.as<int32_t>();
+    l.plan.nodes = l.plan.node_ptr + s.ptr.size();
+    l.plan.ends = reinterpret_cast<const uint32_t *>(l.plan.nodes + s.nodes.size());
+    l.plan.ef_odd = local_ef.p;
+    local = l;
   }
 
   // The records the step kernels read (ElemRecIx, NodeRecIx).
@@ -664,6 +660,7 @@ struct Engine final : EngineBase {
 
   void set_threads(int tpb) override { kernels.tpb_override = tpb; }
   StepLaunch launch_shape(int64_t nsteps) override {
+    ensure_plan(nsteps);
     return step_launch<T>(kernels, m, nsteps, exec_mode, local);
   }
   // Recording the internal force of each launch's last step costs a
@@ -825,6 +822,7 @@ struct Engine final : EngineBase {
       c.last_energy = energy_slots.as<double>() + 5 * (launches & 1);
       c.next_energy = energy_slots.as<double>() + 5 * ((launches + 1) & 1);
       SampleSpec smp = sample_spec();
+      ensure_plan(n);
       auto enqueue = [&]() {
         if (m.lat_energy) DL_CUDA(cudaMemsetAsync(m.lat_energy, 0, lat_energy.bytes, stream));
         cudaError_t e = launch_steps<T>(kernels, m, smp, c, exec_mode, barrier.as<GridBarrier>(), local, stream);
@@ -2324,9 +2322,11 @@ DL_API int dl_jit_check(const dl_model_desc *desc, int precision, size_t *cubin_
     if (ok) {  // and the adjoint kernels of the same model
       const std::string acode = dl::emitYieldAdjPolicy(hl->yield_expr, hl->grad_exprs, precision == DL_MIXED,
                                                        "__device__");
-      ok = dl::jit_compile_adjoint(acode, precision == DL_MIXED, &cubin, &lowered, &l);
-      bytes += ok ? cubin.size() : 0;
+      ok = dl::jit_compile_adjoint(acode, precision == DL_MIXED, &adj, &l);
     }
+    size_t bytes = 0;
+    for (const auto *set : {&step, &adj})
+      for (const dl::JitKernel &k : *set) bytes += k.cubin.size();
     if (cubin_bytes) *cubin_bytes = ok ? bytes : 0;
   });
   if (log && log_size) {
