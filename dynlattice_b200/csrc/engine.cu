@@ -2315,10 +2315,8 @@ DL_API int dl_jit_check(const dl_model_desc *desc, int precision, size_t *cubin_
     auto hl = dl::build_lattice(*desc, precision == DL_MIXED);
     if (!hl->plastic) throw std::invalid_argument("runtime compilation applies to elastoplastic lattices");
     const std::string code = dl::emitYieldPolicy(hl->yield_expr, hl->grad_exprs, precision == DL_MIXED);
-    std::vector<char> cubin;
-    std::vector<std::string> lowered;
-    ok = dl::jit_compile(code, precision == DL_MIXED, &cubin, &lowered, &l);
-    size_t bytes = ok ? cubin.size() : 0;
+    std::vector<dl::JitKernel> step, adj;
+    ok = dl::jit_compile(code, precision == DL_MIXED, &step, &l);
     if (ok) {  // and the adjoint kernels of the same model
       const std::string acode = dl::emitYieldAdjPolicy(hl->yield_expr, hl->grad_exprs, precision == DL_MIXED,
                                                        "__device__");

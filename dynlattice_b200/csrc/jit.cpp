@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <nvrtc.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <fstream>
@@ -12,6 +14,7 @@
 #include <mutex>
 #include <sstream>
 #include <sys/stat.h>
+#include <thread>
 #include <vector>
 
 #include "jit_sources.inc"  // kJitHeaderNames / kJitHeaders (generated from the .cuh files)
@@ -20,10 +23,8 @@ namespace dl {
 
 namespace {
 
-constexpr int kNames = 12;
-
 struct Entry {
-  cudaLibrary_t lib = nullptr;
+  std::vector<cudaLibrary_t> libs;
   KernelSet ks;
 };
 
@@ -69,11 +70,10 @@ bool read_file(const std::string &path, std::vector<char> &out) {
 
 namespace {
 
-// compile `src` (which includes the embedded headers) for sm_100a and lower
-// the kernel name expressions; results cached on disk by content hash
-bool compile_generic(const std::string &src, const std::vector<std::string> &names, bool fp32,
-                     const std::string &tag, std::vector<char> *cubin, std::vector<std::string> *lowered,
-                     std::string *log) {
+// compile one kernel (a name expression) of `src`, which includes the embedded
+// headers, for sm_100a; results cached on disk by content hash
+bool compile_kernel(const std::string &src, const std::string &name, bool fp32, const std::string &tag,
+                    JitKernel *out, std::string *log) {
   const char *T = fp32 ? "float" : "double";
   // the FP32 variant uses approximate (not correctly rounded) division and
   // square root; transcendentals stay accurate (small rotation angles need a
@@ -83,11 +83,10 @@ bool compile_generic(const std::string &src, const std::vector<std::string> &nam
   const char *opts64[] = {"-arch=sm_100a", "-std=c++17", "-DNDEBUG"};
   const char *const *opts = fp32 ? opts32 : opts64;
   const int nopts = fp32 ? 6 : 3;
-  const int nk = static_cast<int>(names.size());
   int nv_major = 0, nv_minor = 0;
   nvrtcVersion(&nv_major, &nv_minor);
   std::string full = src + (fp32 ? "|approx-div-sqrt" : "");
-  for (auto &n : names) full += "|" + n;
+  full += "|" + name;
   for (size_t i = 0; i < sizeof(kJitHeaders) / sizeof(kJitHeaders[0]); ++i) full += kJitHeaders[i];
   char hbuf[64];
   std::snprintf(hbuf, sizeof hbuf, "%016llx_%d_%d_%s", static_cast<unsigned long long>(fnv1a(full)), nv_major,
@@ -95,13 +94,12 @@ bool compile_generic(const std::string &src, const std::vector<std::string> &nam
   const std::string dir = cache_dir();
   const std::string cubin_path = dir + "/" + tag + "_" + hbuf + ".cubin";
   const std::string names_path = dir + "/" + tag + "_" + hbuf + ".names";
-  lowered->assign(nk, "");
   {
     std::vector<char> nb;
-    if (read_file(cubin_path, *cubin) && read_file(names_path, nb)) {
+    if (read_file(cubin_path, out->cubin) && read_file(names_path, nb)) {
       std::stringstream ns(std::string(nb.begin(), nb.end()));
-      for (int i = 0; i < nk; ++i) std::getline(ns, (*lowered)[i]);
-      if (!(*lowered)[nk - 1].empty()) return true;
+      std::getline(ns, out->lowered);
+      if (!out->lowered.empty()) return true;
     }
   }
   nvrtcProgram prog;
@@ -110,7 +108,7 @@ bool compile_generic(const std::string &src, const std::vector<std::string> &nam
     if (log) *log = "nvrtcCreateProgram failed";
     return false;
   }
-  for (auto &n : names) nvrtcAddNameExpression(prog, n.c_str());
+  nvrtcAddNameExpression(prog, name.c_str());
   nvrtcResult rc = nvrtcCompileProgram(prog, nopts, opts);
   if (rc != NVRTC_SUCCESS) {
     size_t ls = 0;
@@ -123,26 +121,80 @@ bool compile_generic(const std::string &src, const std::vector<std::string> &nam
   }
   size_t cs = 0;
   nvrtcGetCUBINSize(prog, &cs);
-  cubin->resize(cs);
-  nvrtcGetCUBIN(prog, cubin->data());
-  for (int i = 0; i < nk; ++i) {
-    const char *ln = nullptr;
-    nvrtcGetLoweredName(prog, names[i].c_str(), &ln);
-    (*lowered)[i] = ln ? ln : "";
-  }
+  out->cubin.resize(cs);
+  nvrtcGetCUBIN(prog, out->cubin.data());
+  const char *ln = nullptr;
+  nvrtcGetLoweredName(prog, name.c_str(), &ln);
+  out->lowered = ln ? ln : "";
   nvrtcDestroyProgram(&prog);
   // best-effort disk cache (atomic rename)
   mkdirs(dir);
   {
     std::ofstream fc(cubin_path + ".tmp", std::ios::binary);
-    fc.write(cubin->data(), static_cast<std::streamsize>(cubin->size()));
+    fc.write(out->cubin.data(), static_cast<std::streamsize>(out->cubin.size()));
   }
   {
     std::ofstream fn(names_path + ".tmp");
-    for (auto &l : *lowered) fn << l << "\n";
+    fn << out->lowered << "\n";
   }
   std::rename((cubin_path + ".tmp").c_str(), cubin_path.c_str());
   std::rename((names_path + ".tmp").c_str(), names_path.c_str());
+  return true;
+}
+
+// Each kernel is a program of its own, and the programs are compiled at the same
+// time: twelve step kernels take 30 s one after another and 7 s on eight cores.
+bool compile_kernels(const std::string &src, const std::vector<std::string> &names, bool fp32,
+                     const std::string &tag, std::vector<JitKernel> *out, std::string *log) {
+  const size_t n = names.size();
+  out->assign(n, JitKernel{});
+  std::vector<std::string> logs(n);
+  std::vector<char> ok(n, 0);
+  std::atomic<size_t> next{0};
+  auto work = [&] {
+    for (size_t i; (i = next.fetch_add(1)) < n;) {
+      try {
+        ok[i] = compile_kernel(src, names[i], fp32, tag, &(*out)[i], &logs[i]);
+      } catch (...) {  // out of memory: not ok
+      }
+    }
+  };
+  std::vector<std::thread> helpers;
+  helpers.reserve(n);
+  const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+  try {
+    while (helpers.size() + 1 < std::min(n, cores)) helpers.emplace_back(work);
+  } catch (const std::exception &) {  // no more threads: those there are do the work
+  }
+  work();
+  for (std::thread &t : helpers) t.join();
+  for (size_t i = 0; i < n; ++i) {
+    if (ok[i]) continue;
+    if (log) *log = logs[i].empty() ? "runtime compilation ran out of memory" : logs[i];
+    return false;
+  }
+  return true;
+}
+
+// Loads compiled kernels; false (with a message) when one cannot be.
+bool load_kernels(const std::vector<JitKernel> &jk, std::vector<cudaLibrary_t> *libs, std::vector<const void *> *k,
+                  std::string *log) {
+  for (const JitKernel &j : jk) {
+    cudaLibrary_t lib = nullptr;
+    cudaKernel_t kernel = nullptr;
+    if (cudaLibraryLoadData(&lib, j.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess) {
+      cudaGetLastError();
+      if (log) *log = "cudaLibraryLoadData failed";
+      return false;
+    }
+    libs->push_back(lib);
+    if (cudaLibraryGetKernel(&kernel, lib, j.lowered.c_str()) != cudaSuccess) {
+      cudaGetLastError();
+      if (log) *log = "cudaLibraryGetKernel failed for " + j.lowered;
+      return false;
+    }
+    k->push_back(reinterpret_cast<const void *>(kernel));
+  }
   return true;
 }
 
@@ -158,12 +210,11 @@ bool device_is_sm100(std::string *log) {
   return true;
 }
 
-std::map<std::string, std::pair<cudaLibrary_t, AdjKernels>> g_adj_cache;
+std::map<std::string, AdjKernels> g_adj_cache;
 
 }  // namespace
 
-bool jit_compile(const std::string &policy_source, bool fp32, std::vector<char> *cubin,
-                 std::vector<std::string> *lowered, std::string *log) {
+bool jit_compile(const std::string &policy_source, bool fp32, std::vector<JitKernel> *out, std::string *log) {
   const char *T = fp32 ? "float" : "double";
   const std::string src = "#include \"milne.cuh\"\n#include \"local.cuh\"\nnamespace dl {\n" + policy_source + "}\n";
   const std::vector<std::string> names = {
@@ -179,16 +230,16 @@ bool jit_compile(const std::string &policy_source, bool fp32, std::vector<char> 
       std::string("&dl::k_persistent<") + T + ", dl::YieldJit, false, true>",
       std::string("&dl::k_local<") + T + ", dl::YieldJit, 1>",
       std::string("&dl::k_local<") + T + ", dl::YieldJit, 2>"};
-  return compile_generic(src, names, fp32, "step", cubin, lowered, log);
+  return compile_kernels(src, names, fp32, "step", out, log);
 }
 
-bool jit_compile_adjoint(const std::string &adj_policy_source, bool fp32, std::vector<char> *cubin,
-                         std::vector<std::string> *lowered, std::string *log) {
+bool jit_compile_adjoint(const std::string &adj_policy_source, bool fp32, std::vector<JitKernel> *out,
+                         std::string *log) {
   const char *T = fp32 ? "float" : "double";
   const std::string src = "#include \"adjoint_kernels.cuh\"\nnamespace dl {\n" + adj_policy_source + "}\n";
   const std::vector<std::string> names = {std::string("&dl::k_adj_node<") + T + ">",
                                           std::string("&dl::k_adj_elem<") + T + ", dl::YieldAdj>"};
-  return compile_generic(src, names, fp32, "adjoint", cubin, lowered, log);
+  return compile_kernels(src, names, fp32, "adjoint", out, log);
 }
 
 const AdjKernels *jit_adjoint_kernels(const std::string &adj_policy_source, bool fp32, std::string *log) {
@@ -198,29 +249,15 @@ const AdjKernels *jit_adjoint_kernels(const std::string &adj_policy_source, bool
   cudaGetDevice(&dev);
   const std::string key = std::string(fp32 ? "f|" : "d|") + std::to_string(dev) + "|" + adj_policy_source;
   auto it = g_adj_cache.find(key);
-  if (it != g_adj_cache.end()) return &it->second.second;
-  std::vector<char> cubin;
-  std::vector<std::string> lowered;
-  if (!jit_compile_adjoint(adj_policy_source, fp32, &cubin, &lowered, log)) return nullptr;
-  cudaLibrary_t lib = nullptr;
-  if (cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess) {
-    cudaGetLastError();
-    if (log) *log = "cudaLibraryLoadData failed";
-    return nullptr;
-  }
-  cudaKernel_t k[2];
-  for (int i = 0; i < 2; ++i)
-    if (cudaLibraryGetKernel(&k[i], lib, lowered[i].c_str()) != cudaSuccess) {
-      cudaGetLastError();
-      if (log) *log = "cudaLibraryGetKernel failed for " + lowered[i];
-      return nullptr;
-    }
-  AdjKernels ak;
-  ak.node = reinterpret_cast<const void *>(k[0]);
-  ak.elem = reinterpret_cast<const void *>(k[1]);
-  auto &slot = g_adj_cache[key];
-  slot = {lib, ak};
-  return &slot.second;
+  if (it != g_adj_cache.end()) return &it->second;
+  std::vector<JitKernel> jk;
+  std::vector<cudaLibrary_t> libs;  // loaded until the process ends
+  std::vector<const void *> k;
+  if (!jit_compile_adjoint(adj_policy_source, fp32, &jk, log) || !load_kernels(jk, &libs, &k, log)) return nullptr;
+  AdjKernels &ak = g_adj_cache[key];
+  ak.node = k[0];
+  ak.elem = k[1];
+  return &ak;
 }
 
 const KernelSet *jit_kernels(const std::string &policy_source, bool fp32, std::string *log) {
@@ -231,34 +268,22 @@ const KernelSet *jit_kernels(const std::string &policy_source, bool fp32, std::s
   const std::string key = std::string(fp32 ? "f|" : "d|") + std::to_string(dev) + "|" + policy_source;
   auto it = g_cache.find(key);
   if (it != g_cache.end()) return &it->second->ks;
-  std::vector<char> cubin;
-  std::vector<std::string> lowered;
-  if (!jit_compile(policy_source, fp32, &cubin, &lowered, log)) return nullptr;
+  std::vector<JitKernel> jk;
+  std::vector<const void *> k;
   auto e = std::make_unique<Entry>();
-  if (cudaLibraryLoadData(&e->lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess) {
-    cudaGetLastError();
-    if (log) *log = "cudaLibraryLoadData failed";
-    return nullptr;
-  }
-  cudaKernel_t k[kNames];
-  for (int i = 0; i < kNames; ++i)
-    if (cudaLibraryGetKernel(&k[i], e->lib, lowered[i].c_str()) != cudaSuccess) {
-      cudaGetLastError();
-      if (log) *log = "cudaLibraryGetKernel failed for " + lowered[i];
-      return nullptr;
-    }
-  e->ks.persistent = reinterpret_cast<const void *>(k[0]);
-  e->ks.element = reinterpret_cast<const void *>(k[1]);
-  e->ks.node = reinterpret_cast<const void *>(k[2]);
-  e->ks.internal_force = reinterpret_cast<const void *>(k[3]);
-  e->ks.gather = reinterpret_cast<const void *>(k[4]);
-  e->ks.persistent_x = reinterpret_cast<const void *>(k[5]);
-  e->ks.element_x = reinterpret_cast<const void *>(k[6]);
-  e->ks.node_x = reinterpret_cast<const void *>(k[7]);
-  e->ks.milne = reinterpret_cast<const void *>(k[8]);
-  e->ks.persistent1 = reinterpret_cast<const void *>(k[9]);
-  e->ks.local[0] = reinterpret_cast<const void *>(k[10]);
-  e->ks.local[1] = reinterpret_cast<const void *>(k[11]);
+  if (!jit_compile(policy_source, fp32, &jk, log) || !load_kernels(jk, &e->libs, &k, log)) return nullptr;
+  e->ks.persistent = k[0];
+  e->ks.element = k[1];
+  e->ks.node = k[2];
+  e->ks.internal_force = k[3];
+  e->ks.gather = k[4];
+  e->ks.persistent_x = k[5];
+  e->ks.element_x = k[6];
+  e->ks.node_x = k[7];
+  e->ks.milne = k[8];
+  e->ks.persistent1 = k[9];
+  e->ks.local[0] = k[10];
+  e->ks.local[1] = k[11];
   e->ks.local_threads = fp32 ? 320 : 256;  // LocalThreads<T>
   e->ks.full_threads = fp32 ? 320 : 256;  // PersistShape<T, false>::kThreads
   e->ks.full_threads_x = 256;             // PersistShape<T, true>::kThreads

@@ -15,14 +15,18 @@ namespace dl {
 // Returns nullptr with a message in *log when NVRTC is unavailable or fails.
 const KernelSet *jit_kernels(const std::string &policy_source, bool fp32, std::string *log);
 
-// Compile only (no device needed): cubin for sm_100a and the lowered kernel names.
-bool jit_compile(const std::string &policy_source, bool fp32, std::vector<char> *cubin,
-                 std::vector<std::string> *lowered, std::string *log);
+// One compiled kernel: cubin for sm_100a and the kernel's lowered name.
+struct JitKernel {
+  std::vector<char> cubin;
+  std::string lowered;
+};
+// Compile only (no device needed).
+bool jit_compile(const std::string &policy_source, bool fp32, std::vector<JitKernel> *out, std::string *log);
 
 // Adjoint kernels (adjoint_kernels.cuh) with the generated YieldAdj policy
 // (expr.cpp: emitYieldAdjPolicy); same caching as jit_kernels.
 const AdjKernels *jit_adjoint_kernels(const std::string &adj_policy_source, bool fp32, std::string *log);
-bool jit_compile_adjoint(const std::string &adj_policy_source, bool fp32, std::vector<char> *cubin,
-                         std::vector<std::string> *lowered, std::string *log);
+bool jit_compile_adjoint(const std::string &adj_policy_source, bool fp32, std::vector<JitKernel> *out,
+                         std::string *log);
 
 }  // namespace dl
