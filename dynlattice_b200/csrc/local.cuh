@@ -176,8 +176,10 @@ __global__ void __launch_bounds__(LocalThreads<T>::value, Y::kMinBlocks < MB ? Y
       const bool own = id < 0;
       const int4 ptr = *reinterpret_cast<const int4 *>(s_rec + i);
       double f[6] = {0, 0, 0, 0, 0, 0};
-      // the copies are sorted by their number of slots, so most warps take one path
-      if (__reduce_max_sync(__activemask(), ptr.y - ptr.x) <= 2) sum_ends<2>(ef, ptr.x, ptr.y, f);
+      // the copies are sorted by their number of slots, most first: the first of the
+      // warp's 32 chooses for all of them
+      const int4 most = *reinterpret_cast<const int4 *>(s_rec + (i & ~31));
+      if (most.y - most.x <= 2) sum_ends<2>(ef, ptr.x, ptr.y, f);
       else sum_ends<sizeof(T) == 4 ? 8 : 4>(ef, ptr.x, ptr.y, f);
       double *const r = s_rows + i * row;
       double2 *const r2 = reinterpret_cast<double2 *>(r);

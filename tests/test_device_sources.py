@@ -20,3 +20,10 @@ def test_one_barrier_kernel_leaves_through_its_write_back():
     after = loop[loop.rindex("__syncthreads();"):]
     assert "st32(m.pos + n" in after and "st32(m.rot + n" in after and "m.vel[vel_ix(n, k)]" in after
     assert loop.count("st32(m.pos") == 1
+
+
+def test_no_warp_collective_over_the_threads_that_happen_to_be_together():
+    """__activemask() names the threads that run together just then, not those
+    that take part in a collective."""
+    for f in list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cu")):
+        assert "__activemask" not in _code(f.name), f.name
