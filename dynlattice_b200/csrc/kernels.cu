@@ -214,8 +214,12 @@ StepLaunch step_launch(const KernelSet &ks, const DevModel<T> &m, int64_t nsteps
   const bool solo = ks.tpb_override <= 0 && work <= kSoloWork;
   int tpb = ks.tpb_override > 0 ? ks.tpb_override : threads_for(work);
   if (solo) {
+    // joint pairs, of which a small model can have thousands, take threads up to
+    // 256: FP64, 256 nodes, us per step with 128 threads / 256 / eight blocks of 32:
+    // 32,640 pairs 120 / 65 / 68, some hundred 11.2 / 7.7 / 12
+    const int items = std::max(work, m.n_jpairs), most = m.n_jpairs > 128 ? 256 : 128;
     tpb = 32;
-    while (tpb < work && tpb < 128) tpb *= 2;
+    while (tpb < items && tpb < most) tpb *= 2;
   } else if (tpb == 256) {
     tpb = ext ? ks.full_threads_x : ks.full_threads;
   }
