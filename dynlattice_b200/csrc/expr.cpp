@@ -250,10 +250,14 @@ struct Builder {
     return id;
   }
 
+  // Whole powers as products, in yield functions.  Load scales keep pow: a product
+  // rounds differently, and an expression can cancel all but that difference.
+  bool products = true;
+
   // a^k: whole exponents from 2 to 8 as products (a general pow costs a hundred
   // instructions and more, and a yield function asks for one at every point)
   int power(int a, int k) {
-    if (code[k].op == XO_CONST && code[k].k >= 2.0 && code[k].k <= 8.0 && code[k].k == std::floor(code[k].k)) {
+    if (products && code[k].op == XO_CONST && code[k].k >= 2.0 && code[k].k <= 8.0 && code[k].k == std::floor(code[k].k)) {
       const int e = static_cast<int>(code[k].k);
       const int sq = emit(XO_SQUARE, a);
       if (e <= 3) return e == 2 ? sq : emit(XO_MUL, sq, a);
@@ -277,6 +281,7 @@ struct Builder {
         int a = build(n->kids[0].get());
         int b = build(n->kids[1].get());
         int op = binOps().at(n->op);
+        if (op == XO_POW && code[b].op == XO_CONST && code[b].k == 2.0) return emit(XO_SQUARE, a);
         return op == XO_POW ? power(a, b) : emit(op, a, b);
       }
       case ExprNode::CALL: {
@@ -362,8 +367,11 @@ double evalExpr(const ExprNode *n, const double *v) {
   throw std::runtime_error("bad expression node");
 }
 
-ExprProgram compileExprs(const std::vector<ExprPtr> &exprs) {
+namespace {
+
+ExprProgram compileProgram(const std::vector<ExprPtr> &exprs, bool products) {
   Builder b;
+  b.products = products;
   std::vector<int> outs;
   for (auto &e : exprs) outs.push_back(b.build(e.get()));
   // liveness: last use of every SSA value
@@ -422,6 +430,18 @@ ExprProgram compileExprs(const std::vector<ExprPtr> &exprs) {
   for (int o : outs) p.outputs.push_back(static_cast<uint8_t>(regOf[o]));
   p.n_regs = nregs;
   return p;
+}
+
+}  // namespace
+
+ExprProgram compileExprs(const std::vector<ExprPtr> &exprs) { return compileProgram(exprs, false); }
+
+ExprProgram compileYield(const std::vector<ExprPtr> &exprs) {
+  try {
+    return compileProgram(exprs, true);
+  } catch (const std::runtime_error &) {  // products take more instructions than the program may have
+    return compileProgram(exprs, false);
+  }
 }
 
 namespace {

@@ -42,6 +42,9 @@ double evalExpr(const ExprNode *n, const double *vars);
 
 // Compile several expressions over the same argument vector into one program.
 ExprProgram compileExprs(const std::vector<ExprPtr> &exprs);
+// The same for yield functions: whole powers from 2 to 8 as products where the
+// program has room for them.
+ExprProgram compileYield(const std::vector<ExprPtr> &exprs);
 // Host interpreter of a compiled program (reference for the device one).
 void runProgram(const ExprProgram &p, const double *args, double *out);
 
