@@ -382,7 +382,6 @@ struct LocalPlan {
   const int32_t *node_ptr = nullptr;  // [blocks + 1] runs of nodes
   const int32_t *nodes = nullptr;     // node, sign bit set where this block owns it
   const uint32_t *ends = nullptr;     // [E] the two end nodes as copies of the element's block (16 bits each)
-  void *ef_odd = nullptr;             // T[2E][6]: end-force slots of odd steps (even ones: DevModel::ef)
 };
 
 struct StepCtx {

@@ -347,9 +347,6 @@ struct Engine final : EngineBase {
       m.prec = T(h.prec);
     }
     pack_records();
-    ef.alloc(static_cast<size_t>(E) * 6 * h.nen * sizeof(T));  // one 6-value slot per element node
-    DL_CUDA(cudaMemset(ef.p, 0, ef.bytes));
-    m.ef = ef.as<T>();
     err.alloc(sizeof(uint32_t));
     DL_CUDA(cudaMemset(err.p, 0, err.bytes));
     m.err = err.as<uint32_t>();
@@ -435,77 +432,96 @@ struct Engine final : EngineBase {
       const KernelSet *ks = jit_kernels(code, sizeof(T) == 4, &jit_log);
       if (ks) kernels = *ks;
     }
+    alloc_slots();
     set_sampling(0, {}, 0);
   }
 
   // The one-barrier kernel's share-out of elements and node copies over the
   // blocks.  One block per SM while the elements of a block stay below its
-  // threads, two above that; a model whose copies do not fit keeps the two-barrier
-  // kernels (blocks = 0).  Made by the first run that can use it: a handle that
-  // differentiates, records group output or steps one by one never does, and the
-  // share-out and its slots cost 0.2 ms at 9,900 elements and 2.3 ms at 128,000.
-  LocalLaunch local;
-  DevBuf local_lists, local_ef;
-  bool local_planned = false;
+  // threads, two above that; a model whose copies do not fit, or that uses what
+  // the kernel does not cover, keeps the two-barrier kernels (local.blocks = 0).
+  LocalLaunch local, local_draft;  // in use; without its lists
+  bool local_planned = true;       // nothing (more) to plan
+
+  // Whether all blocks of the draft are resident at once, with `cap` node copies in
+  // the fullest.
+  bool local_fits(LocalLaunch &l, int cap, int recs) {
+    const int most = kernels.local_threads, chunk = l.plan.chunk;
+    l.threads = std::min(most, (std::max(std::min(chunk, most), cap) + 31) / 32 * 32);
+    l.smem = LocalShape<T>::bytes(cap, recs ? chunk : 0, host->G);
+    l.plan.cap = cap;
+    l.plan.recs = recs;
+    int sms = 0;
+    DL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    return static_cast<int64_t>(resident_blocks(l.kernel, l.threads, l.smem)) * sms >= l.blocks;
+  }
+
+  // ints of whole 128-byte lines; where the lists begin, behind two sets of slots
+  static size_t whole_lines(size_t ints) { return (ints + 31) / 32 * 32; }
+  size_t list_offset() const { return whole_lines(static_cast<size_t>(host->E) * 24 * sizeof(T) / 4) * 4; }
+
+  // The end-force slots, 6 values per element end: where the one-barrier kernel may
+  // run two sets of them, and room for its lists behind.
+  void alloc_slots() {
+    const HostLattice &h = *host;
+    const int E = h.E;
+    const size_t set = static_cast<size_t>(E) * 6 * h.nen * sizeof(T);
+    size_t bytes = set;
+    if (!contact_on && !joint_on && kernels.local[0] && !extended_run(m)) {
+      int sms = 0;
+      DL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+      LocalLaunch l;
+      int per_sm = 1, chunk = E;
+      if (std::max(h.N, E) > kSoloWork) {
+        per_sm = E > sms * kernels.local_threads ? 2 : 1;
+        chunk = (E + per_sm * sms - 1) / (per_sm * sms);
+        chunk = std::max(32, (chunk + 7) / 8 * 8);
+      }
+      l.kernel = kernels.local[per_sm - 1];
+      l.blocks = (E + chunk - 1) / chunk;
+      l.plan.chunk = chunk;
+      // every node has a copy in some block: larger models are spared the share-out
+      if (local_fits(l, (h.N + l.blocks - 1) / l.blocks, 0)) {
+        local_draft = l;
+        local_planned = false;
+        bytes = list_offset() + (whole_lines(l.blocks + 1) + whole_lines(2 * static_cast<size_t>(E)) + E) * sizeof(int32_t);
+      }
+    }
+    ef.alloc(bytes);
+    DL_CUDA(cudaMemset(ef.p, 0, set));
+    m.ef = ef.as<T>();
+  }
+
+  // The share-out itself: made by the first run that can use it.  A handle that
+  // differentiates, records group output or steps one by one never does, and it
+  // costs 0.2 ms at 9,900 elements and 1.5 ms at 128,000.
   void ensure_plan(int64_t nsteps) {
-    if (local_planned || nsteps < 2 || exec_mode == EXEC_STREAM || kernels.tpb_override > 0 || !kernels.local[0]) return;
-    if (contact_on || joint_on || extended_run(m)) return;
-    // nothing can be allocated while the caller records a graph: this run takes
-    // the two-barrier kernels
+    if (local_planned || nsteps < 2 || exec_mode == EXEC_STREAM || kernels.tpb_override > 0 || extended_run(m)) return;
+    // not while the caller records a graph, which would keep the copy of host
+    // lists: such a run takes the two-barrier kernels
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (stream && (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
       cudaGetLastError();
       return;
     }
     local_planned = true;
-    try {
-      plan_local();
-    } catch (const CudaError &) {  // no memory for it
-      local = LocalLaunch{};
-    }
-  }
-  void plan_local() {
     const HostLattice &h = *host;
-    const int E = h.E;
-    int sms = 0;
-    DL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int most = kernels.local_threads;
-    int per_sm = 1, chunk = E;
-    if (std::max(h.N, E) > kSoloWork) {
-      per_sm = E > sms * most ? 2 : 1;
-      chunk = (E + per_sm * sms - 1) / (per_sm * sms);
-      chunk = std::max(32, (chunk + 7) / 8 * 8);
-    }
-    const int blocks = (E + chunk - 1) / chunk;
-    LocalLaunch l;
-    l.kernel = kernels.local[per_sm - 1];
-    l.blocks = blocks;
-    // whether blocks of `cap` copies are resident all at once
-    auto fits = [&](int cap, int recs) {
-      l.threads = std::min(most, (std::max(std::min(chunk, most), cap) + 31) / 32 * 32);
-      l.smem = LocalShape<T>::bytes(cap, recs ? chunk : 0, h.G);
-      l.plan.recs = recs;
-      return static_cast<int64_t>(resident_blocks(l.kernel, l.threads, l.smem)) * sms >= blocks;
-    };
-    // every node has a copy in some block: spare larger models the share-out
-    if (!fits((h.N + blocks - 1) / blocks, 0)) return;
+    LocalLaunch l = local_draft;
     LocalShare s;
-    share_nodes(h, chunk, blocks, s);
-    if (s.cap > 0xffff || (!fits(s.cap, 1) && !fits(s.cap, 0))) return;
+    share_nodes(h, l.plan.chunk, l.blocks, s);
+    if (s.cap > 0xffff || (!local_fits(l, s.cap, 1) && !local_fits(l, s.cap, 0))) return;
     share_ends(h, s);
-    // the lists in one array, the second set of end-force slots; on the run's stream
-    std::vector<int32_t> lists(s.ptr);
-    lists.insert(lists.end(), s.nodes.begin(), s.nodes.end());
-    lists.insert(lists.end(), s.ends.begin(), s.ends.end());
-    local_lists.alloc(lists.size() * sizeof(int32_t));
-    local_ef.alloc(static_cast<size_t>(E) * 12 * sizeof(T));
-    DL_CUDA(cudaMemcpyAsync(local_lists.p, lists.data(), local_lists.bytes, cudaMemcpyHostToDevice, stream));
-    l.plan.chunk = chunk;
-    l.plan.cap = s.cap;
-    l.plan.node_ptr = local_lists.as<int32_t>();
-    l.plan.nodes = l.plan.node_ptr + s.ptr.size();
-    l.plan.ends = reinterpret_cast<const uint32_t *>(l.plan.nodes + s.nodes.size());
-    l.plan.ef_odd = local_ef.p;
+    // on the run's stream
+    int32_t *lists = reinterpret_cast<int32_t *>(ef.as<char>() + list_offset());
+    auto put = [&](const auto &v) {
+      int32_t *const p = lists;
+      DL_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
+      lists += whole_lines(v.size());
+      return p;
+    };
+    l.plan.node_ptr = put(s.ptr);
+    l.plan.nodes = put(s.nodes);
+    l.plan.ends = reinterpret_cast<const uint32_t *>(put(s.ends));
     local = l;
   }
 

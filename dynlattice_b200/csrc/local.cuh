@@ -117,9 +117,10 @@ __global__ void __launch_bounds__(LocalThreads<T>::value, Y::kMinBlocks < MB ? Y
   auto rec_scalar = [&](int i, int k) {
     return reinterpret_cast<const T *>(s_rec + (k / Vec16<T>::n) * plan.cap + i)[k % Vec16<T>::n];
   };
+  const size_t set = static_cast<size_t>(m.E) * 12;
   for (int s = 0; s < c.nsteps; ++s) {
     const int64_t step = c.step0 + s + 1;
-    T *const ef = s & 1 ? static_cast<T *>(plan.ef_odd) : m.ef;
+    T *const ef = m.ef + (s & 1) * set;
     const int64_t sidx = sample_index(smp, c, step);
     const bool last = s + 1 == c.nsteps;
     const bool energy = sidx >= 0 || last;

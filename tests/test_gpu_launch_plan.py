@@ -1,5 +1,5 @@
 """The one-barrier kernel's share-out: made by the first run that can use it, left
-out for models that it cannot hold, and the same bits as the two-barrier kernels
+out for models that the kernel cannot hold, and the same bits as the two-barrier kernels
 over its ragged and two-block forms (each case states the launch it expects)."""
 import numpy as np
 import pytest
@@ -17,26 +17,22 @@ def _free():
     return torch.cuda.mem_get_info()[0]
 
 
-def test_share_out_is_made_by_the_run_that_uses_it(gpu):
-    """A handle that is stepped one by one holds one set of end-force slots; the
-    first run of several steps brings the second one."""
+def test_runs_take_no_device_memory(gpu):
+    """The share-out is made by the first run of several steps, in memory that the
+    handle has; a run of another kind before it does not make it."""
     spec = lattices.lattice_impact("bcc", n=20)
-    slots = spec.n_elems * 12 * 8
+    Lattice(spec, DL_PLAIN_FP64).run(2)   # loads the kernels
     g = Lattice(spec, DL_PLAIN_FP64)
+    g.set_group_output(True)
     g.run(1)
-    g.set_group_output(True)   # the extended kernels: no share-out either
     g.run(3)
     g.set_group_output(False)
-    g.run(1)
-    g.synchronize()
     before = _free()
-    g.run(2)
+    assert g.launch_shape(2)["kernel"] == "one_barrier"
+    for n in (1, 2, 3):
+        g.run(n)
     g.synchronize()
-    used = before - _free()
-    assert used >= slots
-    g.run(3)
-    g.synchronize()
-    assert before - _free() == used
+    assert _free() == before
 
 
 # topology, cells, elements per strut, Gauss points, plastic, precision; blocks
