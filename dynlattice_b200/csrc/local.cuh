@@ -167,7 +167,21 @@ __global__ void __launch_bounds__(LocalThreads<T>::value, Y::kMinBlocks < MB ? Y
 #pragma unroll
       for (int k = 0; k < 3; ++k) s_pre[(6 + k) * plan.cap + i] = np.c[k];
     }
-    if (!grid_wait(bar, bs, word, m.err)) break;
+    if (!grid_wait(bar, bs, word, m.err)) {
+      // the owned copies go back here too: the state is then, as after the
+      // two-barrier kernels, at most a phase or two behind the history, and not the
+      // launch's first.  (One write-back behind the loop costs the FP64 kernel 2 % of
+      // a step, in registers.)
+      for (int i = tid; i < nn; i += nt) {
+        if (s_id[i] >= 0) continue;
+        const int n = s_id[i] & 0x7fffffff;
+        const double *const r = s_rows + i * row;
+        st32(m.pos + n, r[4], r[5], r[6], 0.0);
+        st32(m.rot + n, r[0], r[1], r[2], r[3]);
+        for (int k = 0; k < 6; ++k) m.vel[vel_ix(n, k)] = r[8 + k];
+      }
+      return;
+    }
     // ---- node phase
     NodeOut out;
     out.last_step = c.step0 + c.nsteps;
@@ -204,20 +218,14 @@ __global__ void __launch_bounds__(LocalThreads<T>::value, Y::kMinBlocks < MB ? Y
       r2[4] = make_double2(st.v[0], st.v[1]);
       r2[5] = make_double2(st.v[2], st.v[3]);
       r2[6] = make_double2(st.v[4], st.v[5]);
+      if (last && own) {
+        st32(m.pos + n, st.x.x, st.x.y, st.x.z, 0.0);
+        st32(m.rot + n, st.R.w, st.R.x, st.R.y, st.R.z);
+        for (int k = 0; k < 6; ++k) m.vel[vel_ix(n, k)] = st.v[k];
+      }
     }
     add_node_sums<T>(smp, c, step, sidx, last, energy, out);
     __syncthreads();  // the copies, before the next element phase reads them
-  }
-  // The owned copies go back (each thread its own).  Also where the barrier gave
-  // up: the state is then, as after the two-barrier kernels, at most a phase or two
-  // behind the history, and not the launch's first.
-  for (int i = tid; i < nn; i += nt) {
-    if (s_id[i] >= 0) continue;
-    const int n = s_id[i] & 0x7fffffff;
-    const double *const r = s_rows + i * row;
-    st32(m.pos + n, r[4], r[5], r[6], 0.0);
-    st32(m.rot + n, r[0], r[1], r[2], r[3]);
-    for (int k = 0; k < 6; ++k) m.vel[vel_ix(n, k)] = r[8 + k];
   }
 }
 

@@ -9,17 +9,17 @@ def _code(name):
     return re.sub(r"//.*", "", (CSRC / name).read_text())
 
 
-def test_one_barrier_kernel_leaves_through_its_write_back():
-    """A barrier wait that runs out ends the step loop; the block then writes its
-    nodes' state back like after the last step."""
+def test_one_barrier_kernel_writes_back_where_its_barrier_gives_up():
+    """A block whose barrier wait runs out writes its nodes' state back, like after
+    the last step, before it returns."""
     body = _code("local.cuh")
     body = body[body.index("k_local("):]
     loop = body[body.index("for (int s = 0; s < c.nsteps"):]
-    assert "return" not in re.sub(r"return reinterpret_cast", "", loop)
-    assert re.search(r"if \(!grid_wait\([^;]*\)\) break;", loop)
-    after = loop[loop.rindex("__syncthreads();"):]
-    assert "st32(m.pos + n" in after and "st32(m.rot + n" in after and "m.vel[vel_ix(n, k)]" in after
-    assert loop.count("st32(m.pos") == 1
+    give_up = loop[loop.index("if (!grid_wait("):]
+    give_up = give_up[:give_up.index("return;")]
+    for part in (give_up, loop[loop.index("if (last && own)"):]):
+        assert "st32(m.pos + n" in part and "st32(m.rot + n" in part and "m.vel[vel_ix(n, k)]" in part
+    assert loop.count("return;") == 1
 
 
 def test_no_warp_collective_over_the_threads_that_happen_to_be_together():
