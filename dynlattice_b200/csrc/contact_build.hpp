@@ -154,8 +154,9 @@ struct JointList {
   void build(const double4 *pos);
 };
 
-// max_n |v_n| (translations, [6][N] layout) through `scratch` (one word); synchronises `stream`
-// Largest speed of a node, and how far one is from the positions x (null: 0).
+// Largest speed of a node (translations; velocities as DevModel::vel), and how far
+// one has come from the positions x ([N][3]; null: 0).  Clears and writes two words
+// of `scratch`, and synchronises `stream`.
 struct NodeMotion {
   double speed = 0.0, moved = 0.0;
 };

@@ -27,7 +27,8 @@
 //   ediss double[G][E]  dissipated energy per Gauss point
 //   eslot int2[E]       slots of the element's two ends
 //   ef    T[2E][6]      end forces in node-ordered slots: an element writes
-//                       its two records, a node sums its contiguous run
+//                       its two records, a node sums its contiguous run; a second
+//                       set behind it for models of the one-barrier kernel
 // Plain-data device types of the engine, shared by the ahead-of-time build
 // (nvcc) and the runtime-compiled kernels (NVRTC): no standard headers here.
 #pragma once
@@ -345,7 +346,7 @@ struct AdjCtx {
   double *lv = nullptr;     // [6][N] velocity adjoint
   double *lf = nullptr;     // [6][N] adjoint of the internal force of the step
   double *aslot = nullptr;  // [2E][6] element-end contributions (translation 3, rotation 3)
-  double *lep = nullptr;    // [G*6][E] history adjoints (component-major, as DevModel::ep)
+  double *lep = nullptr;    // [G*6][E] history adjoints (component-major)
   double *lal = nullptr;    // [G*nh][E]
   double *lepsc = nullptr;  // [G*6][E]
   double *lC = nullptr;     // [6][E] accumulated adjoint of the section stiffness
@@ -371,6 +372,12 @@ struct GridBarrier {
   unsigned int phantom;
   unsigned int abort;
   unsigned int limit_us;
+};
+
+// Most threads of a block of the one-barrier step kernel.
+template <class T>
+struct LocalThreads {
+  static constexpr int value = sizeof(T) == 4 ? 320 : 256;
 };
 
 // Which elements and nodes each block of a launch takes in the

@@ -894,7 +894,6 @@ struct Engine final : EngineBase {
     if (h.scales.size() > static_cast<size_t>(kMilneMaxScales))
       throw dl::UnsupportedError("MilneDevice takes at most 32 load-scale functions");
     const int N = h.N, E = h.E, G = h.G;
-    const int nhA = std::max(1, h.nh);
     if (integ.kind != DL_INTEG_MILNE) {
       mi_pos.alloc(static_cast<size_t>(N) * sizeof(double4));
       mi_rot.alloc(static_cast<size_t>(N) * sizeof(double4));

@@ -284,7 +284,7 @@ const KernelSet *jit_kernels(const std::string &policy_source, bool fp32, std::s
   e->ks.persistent1 = k[9];
   e->ks.local[0] = k[10];
   e->ks.local[1] = k[11];
-  e->ks.local_threads = fp32 ? 320 : 256;  // LocalThreads<T>
+  e->ks.local_threads = fp32 ? LocalThreads<float>::value : LocalThreads<double>::value;
   e->ks.full_threads = fp32 ? 320 : 256;  // PersistShape<T, false>::kThreads
   e->ks.full_threads_x = 256;             // PersistShape<T, true>::kThreads
   set_persistent_caps(e->ks);

@@ -66,14 +66,9 @@ struct LocalEnds {
   }
 };
 
-// Most threads of a block.  MB: blocks per SM that the kernel's registers leave
-// room for.  Models of at most a block per SM take the MB = 1 kernel, whose 204
-// (255) registers a thread spill nothing.
-template <class T>
-struct LocalThreads {
-  static constexpr int value = sizeof(T) == 4 ? 320 : 256;
-};
-
+// MB: blocks per SM that the kernel's registers leave room for.  Models of at most
+// a block per SM take the MB = 1 kernel: 168 (FP64 255) registers a thread and half
+// the spills of MB = 2, which has 96 (128): 456 against 820 bytes (552 against 1,180).
 template <class T, class Y, int MB>
 __global__ void __launch_bounds__(LocalThreads<T>::value, Y::kMinBlocks < MB ? Y::kMinBlocks : MB)
     k_local(const __grid_constant__ DevModel<T> m, const __grid_constant__ SampleSpec smp, const StepCtx c,
