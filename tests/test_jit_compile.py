@@ -11,17 +11,26 @@ import pytest
 ROOT = Path(__file__).resolve().parent.parent
 
 SCRIPT = """
-import ctypes as C, json, os, time
+import ctypes as C, json, os, threading, time
 from dynlattice_b200 import lattices
 from dynlattice_b200.engine import load_library
 lib = load_library()
 d = lattices.lattice_impact(n=1).desc()
 n, log = C.c_size_t(), C.create_string_buffer(1 << 16)
-out = []
+tasks = lambda: len(os.listdir("/proc/self/task"))
+done, most = threading.Event(), [0]
+def watch():
+    while not done.wait(0.05):
+        most[0] = max(most[0], tasks())
+w = threading.Thread(target=watch)
+w.start()
+before, out = tasks(), []
 for _ in range(2):
-    wall, cpu = time.perf_counter(), time.process_time()
+    wall = time.perf_counter()
     rc = lib.dl_jit_check(C.byref(d), int(os.environ["PREC"]), C.byref(n), log, C.c_size_t(1 << 16))
-    out.append([rc, n.value, time.perf_counter() - wall, time.process_time() - cpu])
+    out.append([rc, n.value, time.perf_counter() - wall, most[0] - before])
+done.set()
+w.join()
 print(json.dumps(out))
 """
 
@@ -38,7 +47,5 @@ def test_kernels_compile_side_by_side(tmp_path, precision):
         files = [p for p in tmp_path.iterdir() if p.suffix == ext]
         assert len([p for p in files if p.name.startswith("step_")]) == 12
         assert len([p for p in files if p.name.startswith("adjoint_")]) == 2
-    cores = len(os.sched_getaffinity(0))
-    if cores >= 4:
-        assert first[2] < 0.8 * first[3]   # wall against CPU time: several threads at work
+    assert first[3] >= min(len(os.sched_getaffinity(0)), 12) - 1   # threads beside the caller's
     assert second[2] < 0.2 * first[2]      # from the cache
